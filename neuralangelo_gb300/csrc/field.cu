@@ -167,60 +167,184 @@ __device__ __forceinline__ void scatter_add(float* dst, const float* v) {
 
 // ---------------------------------------------------------------------------
 // hash-grid gather and table-gradient scatter as their own kernels: one thread
-// per (row, level) / (sample, level, corner) keeps thousands of independent
-// loads and atomics in flight, which the tensor-core kernels (one CTA of eight
-// warps per SM) cannot.
+// per (sample, level) keeps thousands of independent loads and atomics in flight,
+// which the tensor-core kernels (one CTA of eight warps per SM) cannot.
+
+// Two float32 lanes in one register pair: fma.rn.f32x2 rounds each lane as fmaf does and
+// takes half the issue slots.
+__device__ __forceinline__ uint64_t pack_f32x2(float lo, float hi) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void unpack_f32x2(uint64_t v, float& lo, float& hi) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+
+// one table row of F fp16 features
+template <int F>
+struct TableRow {
+    uint32_t u[F / 2];
+    __device__ __forceinline__ void load(const __half* row) {
+        if constexpr (F == 8) {
+            const uint4 q = __ldg(reinterpret_cast<const uint4*>(row));
+            u[0] = q.x; u[1] = q.y; u[2] = q.z; u[3] = q.w;
+        } else if constexpr (F == 4) {
+            const uint2 q = __ldg(reinterpret_cast<const uint2*>(row));
+            u[0] = q.x; u[1] = q.y;
+        } else {
+            u[0] = __ldg(reinterpret_cast<const uint32_t*>(row));
+        }
+    }
+    // v += w * row, each feature one fmaf
+    __device__ __forceinline__ void fma(float w, uint64_t* v) const {
+        const uint64_t ww = pack_f32x2(w, w);
+#pragma unroll
+        for (int i = 0; i < F / 2; ++i) {
+            const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&u[i]));
+            v[i] = fma_f32x2(ww, pack_f32x2(f.x, f.y), v[i]);
+        }
+    }
+};
+
+// The level table in shared memory: lanes of a warp sit on different levels, and a
+// lane-dependent index into the kernel parameters is serialised per level.
+__device__ __forceinline__ void stage_levels(const gbsdf_grid& g, LevelDesc* lv_s, int active) {
+    for (int l = threadIdx.x; l < active; l += blockDim.x) lv_s[l] = level_desc(g, l);
+}
+
+// grid cell and fraction of a point on one level
+struct GridCell {
+    uint32_t b[3];
+    float f[3];
+};
+__device__ __forceinline__ GridCell grid_cell(float scale, const float* x) {
+    GridCell g;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) grid_pos(scale, to_unit(x[k]), g.b[k], g.f[k]);
+    return g;
+}
+
+// The (lane, evaluation) pairs of a warp named in each lane's `mask` (bit e), packed into
+// list (lane << 3 | e); returns their number.  EVALS <= 8.
+template <int EVALS>
+__device__ __forceinline__ int warp_pack_evals(uint32_t mask, uint8_t* list, int lane) {
+    const int n = __popc(mask);
+    int at = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, at, o);
+        if (lane >= o) at += v;
+    }
+    const int total = __shfl_sync(0xffffffffu, at, 31);
+    at -= n;
+#pragma unroll
+    for (int e = 1; e < EVALS; ++e)
+        if (mask & (1u << e)) list[at++] = (uint8_t)(lane << 3 | e);
+    __syncwarp();
+    return total;
+}
 
 // x0ext row t*126 + r (r = e*18 + sl) of every tile: the features of level l in
-// columns [l F, l F + F) as fp16 hi and, at K0 + 16 + l F, the fp16 residual lo;
-// the level-0 thread also writes the 16-column tail after the hi features and
-// zeroes the padding columns.  Rows of samples past the end are zeros.
-// Six blocks per SM (at most 40 registers): the gather waits on L2 latency, and the
-// extra resident warps keep more corner loads in flight.
+// columns [l F, l F + F) as fp16 hi and, at K0 + 16 + l F, the fp16 residual lo; then the
+// 16-column tail after the hi features and the zeroed padding columns.  Rows of samples
+// past the end are zeros.
+//
+// One thread per (sample, level), levels fastest, so that a warp's stores of one evaluation
+// cover whole rows.  The taps lie a fraction of a cell from the centre (a quarter at the
+// finest active level, less below it), so most evaluations interpolate the centre's own
+// eight corners: they are loaded once, kept in registers as fp16, and every evaluation
+// in the centre's cell costs arithmetic only.  The evaluations in another cell (about one in
+// nine) are packed across the warp and taken one per lane, so they cost one or two dense
+// passes instead of a divergent one per tap.  Values and order of the products are those of
+// an evaluation that loads its own corners.
+// One thread per (evaluation, level), each loading its own eight corners, was bound by L1
+// (73 %): 2.60 ms for 2.1 M samples x 8 levels, 20.7 ms for 6.3 M samples x 16 levels; this
+// takes 1.34 and 8.1 ms (the rows it writes: 0.63 and 3.5 ms at the copy rate).  Latency
+// bounds it: the corners kept as float32 (120 registers, two blocks per SM) took 2.07 ms, the
+// tap loop unrolled 1.37 ms at two blocks and 1.73 at three, five blocks (spills) 1.75 ms.
+constexpr int GATHER_THREADS = 256;
 template <int F, int TAPS>
-__global__ void __launch_bounds__(256, 6) k_field_gather(FieldParams p, int64_t ntiles) {
+__global__ void __launch_bounds__(GATHER_THREADS, 4) k_field_gather(FieldParams p, int64_t ntiles) {
     constexpr int EVALS = TapTile<TAPS>::EVALS, SPT = TapTile<TAPS>::SPT;
+    __shared__ LevelDesc lv_s[GBSDF_MAX_LEVELS];
+    __shared__ uint8_t list_s[GATHER_THREADS / 32][32 * TAPS];
     const int A = p.active, K0 = p.K0, KX = 2 * K0 + 16;
+    stage_levels(p.grid, lv_s, A);
+    __syncthreads();
     // 32-bit index arithmetic: the launcher checks rows * A < 2^32
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t rows = (uint32_t)(ntiles * (SPT * EVALS));
-    if (i >= rows * (uint32_t)A) return;
-    // thread order (tile, sample, evaluation, level): the 7 evaluations of a sample are
-    // neighbouring threads, so at coarse levels (same cell for all taps) their corner
-    // rows come from L1; the output row is t * 126 + e * 18 + sl
-    const uint32_t q = i / (uint32_t)A;
-    const int l = (int)(i - q * (uint32_t)A);
-    const uint32_t se = q / EVALS;                   // tile-major sample slot
-    const int e = (int)(q - se * EVALS);
-    const int64_t t = se / SPT;
-    const int sl = (int)(se - (uint32_t)t * SPT);
-    const uint32_t grow = (uint32_t)t * (SPT * EVALS) + e * SPT + sl;
-    const int64_t s = t * SPT + sl;
-    __half* dst = (__half*)p.x0ext + (int64_t)grow * KX;     // 64-bit: rows * KX can exceed 2^32
-    float v[F], lo[F];
-    float x[3] = {0.f, 0.f, 0.f};
-    const bool live = s < p.Ns;
+    const uint32_t slots = (uint32_t)(ntiles * SPT);      // sample slots, tile-major
+    const bool in = i < slots * (uint32_t)A;              // (whole warps go on: they pack their crossings together)
+    const uint32_t se = in ? i / (uint32_t)A : 0u;
+    const int l = in ? (int)(i - se * (uint32_t)A) : 0;
+    const uint32_t t = se / SPT;
+    const uint32_t row0 = t * (SPT * EVALS) + (se - t * SPT);   // evaluation e's row: row0 + e * SPT
+    const bool live = in && (int64_t)se < p.Ns;
+    const int lane = threadIdx.x & 31;
+    __half* const x0 = (__half*)p.x0ext;
+    const __half* const table = (const __half*)p.table;
+
+    auto emit = [&](uint32_t row, int lev, const uint64_t* v) {
+        __half* dst = x0 + (int64_t)row * KX + lev * F;          // 64-bit: rows * KX can exceed 2^32
+        float hi[F], lo[F];
+#pragma unroll
+        for (int k = 0; k < F / 2; ++k) unpack_f32x2(v[k], hi[2 * k], hi[2 * k + 1]);
+#pragma unroll
+        for (int f = 0; f < F; ++f) lo[f] = hi[f] - __half2float(__float2half_rn(hi[f]));
+        write_half_row<F>(reinterpret_cast<uint8_t*>(dst), hi);
+        write_half_row<F>(reinterpret_cast<uint8_t*>(dst + K0 + 16), lo);
+    };
+
+    float c[3] = {0.f, 0.f, 0.f};
+    uint32_t mask = 0;                                    // evaluations outside the centre's cell
     if (live) {
-        float c[3], xu[3];
-        sample_point(p, s, c);
-        eval_point<TAPS>(c, e, p.eps, x);
+        sample_point(p, se, c);
+        const LevelDesc d = lv_s[l];
+        const GridCell g0 = grid_cell(d.scale, c);
+        TableRow<F> home[8];
 #pragma unroll
-        for (int k = 0; k < 3; ++k) xu[k] = to_unit(x[k]);
-        gather_level<F>(p, xu, l, v);
-    } else {
+        for (int k = 0; k < 8; ++k)
+            home[k].load(table + (d.offset + grid_index(d, g0.b[0] + (k & 1), g0.b[1] + ((k >> 1) & 1),
+                                                             g0.b[2] + ((k >> 2) & 1))) * F);
+#pragma unroll 1
+        for (int e = 0; e < EVALS; ++e) {
+            float x[3];
+            eval_point<TAPS>(c, e, p.eps, x);
+            const GridCell g = grid_cell(d.scale, x);
+            if (g.b[0] == g0.b[0] && g.b[1] == g0.b[1] && g.b[2] == g0.b[2]) {
+                uint64_t v[F / 2];
 #pragma unroll
-        for (int f = 0; f < F; ++f) v[f] = 0.0f;
+                for (int k = 0; k < F / 2; ++k) v[k] = 0ull;
+#pragma unroll
+                for (int k = 0; k < 8; ++k) {
+                    const float w = corner_weight(k, g.f[0], g.f[1], g.f[2]);
+                    home[k].fma(w, v);
+                }
+                emit(row0 + e * SPT, l, v);
+            } else {
+                mask |= 1u << e;
+            }
+        }
+    } else if (in) {
+        const uint64_t v[F / 2] = {};
+        for (int e = 0; e < EVALS; ++e) emit(row0 + e * SPT, l, v);
     }
-#pragma unroll
-    for (int f = 0; f < F; ++f) lo[f] = v[f] - __half2float(__float2half_rn(v[f]));
-    write_half_row<F>(reinterpret_cast<uint8_t*>(dst + l * F), v);
-    write_half_row<F>(reinterpret_cast<uint8_t*>(dst + K0 + 16 + l * F), lo);
-    if (l == 0) {
-        // tail (multiplied by w0b's position and bias columns in the forward MMA):
-        // x hi, 1, x lo, 1, x hi, zeros -- w0x x + b0 as fp16 hi/lo products
+    // tail (multiplied by w0b's position and bias columns in the forward MMA): x hi, 1, x lo, 1,
+    // x hi, zeros -- w0x x + b0 as fp16 hi/lo products; lane l of a sample takes evaluations l, l + A, ..
+    for (int e = l; in && e < EVALS; e += A) {
+        __half* dst = x0 + (int64_t)(row0 + e * SPT) * KX;
         float tail[16] = {0.f};
         if (live) {
+            float x[3];
+            eval_point<TAPS>(c, e, p.eps, x);
             tail[0] = x[0]; tail[1] = x[1]; tail[2] = x[2]; tail[3] = 1.0f;
+#pragma unroll
             for (int k = 0; k < 3; ++k) tail[4 + k] = x[k] - __half2float(__float2half_rn(x[k]));
             tail[7] = 1.0f;
             tail[8] = x[0]; tail[9] = x[1]; tail[10] = x[2];
@@ -231,6 +355,35 @@ __global__ void __launch_bounds__(256, 6) k_field_gather(FieldParams p, int64_t 
             dst[c0] = __float2half_rn(0.0f);
             dst[K0 + 16 + c0] = __float2half_rn(0.0f);
         }
+    }
+    uint8_t* list = list_s[threadIdx.x >> 5];
+    const int total = warp_pack_evals<EVALS>(mask, list, lane);
+    for (int k0 = 0; k0 < total; k0 += 32) {
+        const bool on = k0 + lane < total;
+        const int ent = on ? list[k0 + lane] : 0, own = ent >> 3, e = ent & 7;
+        const float oc[3] = {__shfl_sync(0xffffffffu, c[0], own), __shfl_sync(0xffffffffu, c[1], own),
+                             __shfl_sync(0xffffffffu, c[2], own)};
+        const int ol = __shfl_sync(0xffffffffu, l, own);
+        const uint32_t orow = __shfl_sync(0xffffffffu, row0, own);
+        if (!on) continue;
+        float x[3];
+        eval_point<TAPS>(oc, e, p.eps, x);
+        const LevelDesc d = lv_s[ol];
+        const GridCell g = grid_cell(d.scale, x);
+        uint64_t v[F / 2];
+        TableRow<F> r[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+            r[k].load(table + (d.offset + grid_index(d, g.b[0] + (k & 1), g.b[1] + ((k >> 1) & 1),
+                                                             g.b[2] + ((k >> 2) & 1))) * F);
+#pragma unroll
+        for (int f = 0; f < F / 2; ++f) v[f] = 0ull;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const float w = corner_weight(k, g.f[0], g.f[1], g.f[2]);
+            r[k].fma(w, v);
+        }
+        emit(orow + e * SPT, ol, v);
     }
 }
 
@@ -1381,8 +1534,9 @@ static int launch_field(const FieldParams& p, int which, cudaStream_t s) {
         return GBSDF_ERR_UNSUPPORTED;
     }
     if (which & FK_GATHER) {
-        const int64_t items = ntiles * (SPT * EVALS) * p.active;
-        k_field_gather<F, TAPS><<<(unsigned)((items + 255) / 256), 256, 0, s>>>(p, ntiles);
+        const int64_t items = ntiles * SPT * p.active;
+        k_field_gather<F, TAPS><<<(unsigned)((items + GATHER_THREADS - 1) / GATHER_THREADS), GATHER_THREADS, 0, s>>>(
+            p, ntiles);
         if (int st = launch_status("field gather")) return st;
     }
     if (which & FK_MLP_FWD) {
