@@ -93,3 +93,51 @@ def test_gather_rows_match_the_oracle_at_every_evaluation(case):
         np.testing.assert_array_equal(tail[:, 8:11], tail[:, :3])
     assert (got[~live] == 0).all()                        # samples past the end
     assert (got[:, AF:K0] == 0).all() and (got[:, K0 + 16 + AF:] == 0).all()
+
+
+@pytest.mark.parametrize("fixed", [False, True])
+@pytest.mark.parametrize("case", CASES)
+def test_scatter_matches_the_oracle_sum_over_evaluations(case, fixed):
+    f = Field(*case)
+    g = torch.Generator().manual_seed(9)
+    d_enc = torch.randn(f.rows, f.K0, generator=g)
+    scale = 0.37
+    f.keep["d_enc"] = d_enc.to(DEV)
+    f.keep["out"] = out = torch.zeros(f.lay.n_params, device=DEV)
+    f.a.d_enc, f.a.d_table, f.a.d_table_scale = f.keep["d_enc"].data_ptr(), out.data_ptr(), scale
+    if fixed:
+        f.keep["fix"] = torch.zeros(f.lay.n_params, device=DEV, dtype=torch.int64)
+        f.a.d_table_fix = f.keep["fix"].data_ptr()
+    want = np.zeros((f.lay.n_entries, f.F))
+    mag = np.zeros((f.lay.n_entries, f.F))
+    for e in range(f.evals):
+        d = np.zeros((f.n, f.lay.n_levels * f.F))
+        d[:, :f.active * f.F] = d_enc.numpy()[f.row_of(e), :f.active * f.F]
+        want += hg.encode_backward(f.unit[e], d, f.ora, f.active)
+        mag += hg.encode_backward(f.unit[e], np.abs(d), f.ora, f.active)
+    s32 = float(np.float32(scale))
+    for cpt in (0, 2, 4, 8):
+        out.zero_()
+        f.a.scatter_cpt = cpt
+        f.call("gbsdf_field_scatter")
+        got = out.double().cpu().numpy().reshape(-1, f.F)
+        # float32 weights (four roundings) and products, sums in any order of at most
+        # evals * samples terms; 2^-48 steps of the fixed-point form
+        bound = mag * s32 * (f.evals * f.n + 8) * 2.0 ** -24 + 8 * f.evals * f.n * 2.0 ** -48
+        assert (np.abs(got - want * s32) <= bound).all()
+        assert (got[mag == 0] == 0).all()
+
+
+def test_scatter_keeps_a_non_finite_gradient_to_its_own_corners():
+    f = Field(8, 6, 16, 8, 0.9, 40)
+    f.keep["d_enc"] = d_enc = torch.ones(f.rows, f.K0, device=DEV)
+    bad = f.row_of(3)[7]
+    d_enc[bad] = float("inf")
+    f.keep["out"] = out = torch.zeros(f.lay.n_params, device=DEV)
+    f.keep["flag"] = flag = torch.zeros(1, device=DEV)
+    f.a.d_enc, f.a.d_table, f.a.d_table_scale = d_enc.data_ptr(), out.data_ptr(), 1.0
+    f.a.found_inf = flag.data_ptr()
+    f.call("gbsdf_field_scatter")
+    reach = hg.all_indices(f.unit[3][7:8], f.ora, f.active).reshape(-1)
+    hit = ~np.isfinite(out.cpu().numpy().reshape(-1, 8)).all(axis=1)
+    assert flag.item() == 1 and set(np.flatnonzero(hit)) == set(reach.tolist())
