@@ -108,6 +108,24 @@ __device__ __forceinline__ void load_half8(const __half* src, float* v) {
 }
 
 // report a timed-out wait through a device flag the host reads after the launch
+// Named CTA barriers for a subset of the warps (n threads, whole warps; ids 1-15)
+__device__ __forceinline__ void named_barrier_sync(int id, int n) {
+    asm volatile("barrier.cta.sync %0, %1;" ::"r"(id), "r"(n) : "memory");
+}
+// the same, returning whether `v` held on every thread
+__device__ __forceinline__ bool named_barrier_and(int id, int n, bool v) {
+    uint32_t r;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.u32 p, %1, 0;\n\t"
+        "barrier.cta.red.and.pred q, %2, %3, p;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t}"
+        : "=r"(r)
+        : "r"((uint32_t)v), "r"(id), "r"(n)
+        : "memory");
+    return r != 0;
+}
+
 __device__ __forceinline__ void flag_timeout(int* err, int code) {
     if (err) atomicCAS(err, 0, code);
 }

@@ -1422,113 +1422,198 @@ struct SdfPointsArgs {
     float* out;                // [M]
 };
 
+// Warp-specialised, one persistent CTA per SM, two tiles in flight:
+//   warps 0-15   gather: warp w fills rows 32 (w & 3) .. of every fourth level starting at
+//                w >> 2, one lane per row, so the lanes of a warp share their level's constants
+//                and neighbouring points of a lattice row share corners; a buffer is full when
+//                all sixteen have arrived on full[b];
+//   warp 24      issues the tile's MMAs (A: the features' fp16 residuals, then hi; B: W0e) into
+//                one of two TMEM accumulators; their completion (done[b]) frees the
+//                feature buffer and starts the epilogue;
+//   warps 16-23  the epilogue: the position columns, bias, softplus and the head in fp32, one
+//                half of the hidden units per warp; tempty[b] hands the accumulator back.
+// Gather, MMAs and epilogue of one tile used to follow one another in eight warps, so the
+// table's latency stood in every tile.  2.1 M lattice points x 16 levels: 3.79 ms
+// in that form, 1.16 ms in this one; 5.5 M scattered points of a view (four calls) 12.1 and 4.0 ms.
+constexpr int SP_GATHER_WARPS = 16;
+constexpr int SP_EPI_WARPS = 8;
+constexpr int SP_TPB = (SP_GATHER_WARPS + SP_EPI_WARPS + 1) * 32;
+constexpr int SP_XRING = 4;      // points kept for the epilogue: two tiles ahead of the one it may still read
+
+static size_t sdf_points_smem(int K0) {
+    return (size_t)HID * K0 * 2 + 4 * (size_t)TILE_M * K0 * 2 + HID * 20 + 2 * 2 * TILE_M * 4 +
+           SP_XRING * TILE_M * 12 + 6 * 8 + 16;
+}
+
 template <int F>
-__global__ void __launch_bounds__(FIELD_THREADS, 1) k_sdf_points(FieldParams p, SdfPointsArgs q) {
+__global__ void __launch_bounds__(SP_TPB, 1) k_sdf_points(FieldParams p, SdfPointsArgs q) {
     extern __shared__ __align__(1024) uint8_t smem[];
-    const int K0 = p.K0;
-    uint8_t* w_s = smem;
-    uint8_t* a_s = w_s + HID * K0 * 2;
-    uint8_t* a2_s = a_s + TILE_M * K0 * 2;
-    float* w0x_s = reinterpret_cast<float*>(a2_s + TILE_M * K0 * 2);
-    float* b0_s = w0x_s + HID * 3;
-    float* wh_s = b0_s + HID;
-    float* part_s = wh_s + HID;                                 // [2][128]
-    uint64_t* mbar = reinterpret_cast<uint64_t*>(part_s + 2 * TILE_M);
-    uint32_t* tslot = reinterpret_cast<uint32_t*>(mbar + 1);
+    const int K0 = p.K0, A = p.active;
+    const uint32_t a_bytes = (uint32_t)TILE_M * K0 * 2;
+    uint8_t* w_s = smem;                                        // [256 x K0]  W0e
+    uint8_t* a_s = w_s + HID * K0 * 2;                          // [2 buffers][lo, hi][128 x K0]  features
+    float4* wx_s = reinterpret_cast<float4*>(a_s + 4 * a_bytes);   // [256] position columns, bias
+    float* wh_s = reinterpret_cast<float*>(wx_s + HID);         // [256] head
+    float* part_s = wh_s + HID;                                 // [2][2][128] partial head sums
+    float* x_s = part_s + 4 * TILE_M;                           // [SP_XRING][3][128] points
+    uint64_t* full = reinterpret_cast<uint64_t*>(x_s + SP_XRING * 3 * TILE_M);   // [2]
+    uint64_t* done = full + 2;                                  // [2]
+    uint64_t* tempty = done + 2;                                // [2]
+    uint32_t* tslot = reinterpret_cast<uint32_t*>(tempty + 2);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    stage_rows_kmajor(w_s, (const __half*)p.w0e, 0, HID, K0, K0, tid, FIELD_THREADS, HID);
-    for (int i = tid; i < HID * 3; i += FIELD_THREADS) w0x_s[i] = p.w0x[i];
-    for (int i = tid; i < HID; i += FIELD_THREADS) {
-        b0_s[i] = p.b0[i];
-        wh_s[i] = p.whead[i];
-    }
-    for (int i = tid; i < 2 * TILE_M * K0 / 8; i += FIELD_THREADS)
-        reinterpret_cast<uint4*>(a_s)[i] = make_uint4(0, 0, 0, 0);
+    if (A * F < K0)                                             // the padding columns stay zero
+        for (uint32_t i = tid; i < 4 * a_bytes / 16; i += SP_TPB)
+            reinterpret_cast<uint4*>(a_s)[i] = make_uint4(0, 0, 0, 0);
+    umma::fence_proxy_async_smem();
     if (tid == 0) {
-        umma::mbar_init(mbar, 1);
+        for (int b = 0; b < 2; ++b) {
+            umma::mbar_init(&full[b], SP_GATHER_WARPS);
+            umma::mbar_init(&done[b], 2);
+            umma::mbar_init(&tempty[b], SP_EPI_WARPS);
+        }
         umma::fence_mbar_init();
     }
-    if (warp == 0) {
-        umma::tmem_alloc(tslot, HID);
+    if (warp == SP_GATHER_WARPS + SP_EPI_WARPS) {
+        umma::tmem_alloc(tslot, 2 * HID);
         umma::tmem_relinquish();
-    }
-    cp_async_wait_all();
-    __syncthreads();
-    umma::fence_after_sync();
-    const uint32_t tmem = *tslot;
-    const uint32_t idesc = umma::idesc_f16(TILE_M, HID);
-    const uint32_t a_addr = umma::smem_u32(a_s), a2_addr = umma::smem_u32(a2_s), w_addr = umma::smem_u32(w_s);
-    const float bhead = p.bhead[0];
-    const SoftplusK spk = softplus_k(p.beta);
-    const int64_t ntiles = (q.M + TILE_M - 1) / TILE_M;
-    const int qd = warp & 3, half = warp >> 2;
-    const int row = qd * 32 + lane;
-    uint32_t phase = 0;
-    auto point = [&](int64_t m, float* x) {
-        if (q.pts) {
-            x[0] = q.pts[3 * m]; x[1] = q.pts[3 * m + 1]; x[2] = q.pts[3 * m + 2];
-        } else {
-            const int k = (int)(m % q.nz), j = (int)((m / q.nz) % q.ny), i = (int)(m / ((int64_t)q.ny * q.nz));
-            x[0] = q.ax[i]; x[1] = q.ay[j]; x[2] = q.az[k];
-        }
-    };
-    for (int64_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
-        const int64_t m0 = t * TILE_M;
-        for (int i = tid; i < TILE_M * p.active; i += FIELD_THREADS) {
-            const int r = i / p.active, l = i % p.active;
-            const int64_t m = m0 + r;
-            float v[F];
-            if (m < q.M) {
-                float x[3], xu[3];
-                point(m, x);
-#pragma unroll
-                for (int k = 0; k < 3; ++k) xu[k] = to_unit(x[k]);
-                gather_level<F>(p, xu, l, v);
-            } else {
-#pragma unroll
-                for (int f = 0; f < F; ++f) v[f] = 0.0f;
-            }
-            write_tile_features<F>(a_s, a2_s, r, l, K0, v);
-        }
-        umma::fence_proxy_async_smem();
-        __syncthreads();
-        if (tid == 0) {
-            umma::fence_after_sync();
-            issue_tile_mma(tmem, a2_addr, w_addr, K0, idesc);          // residuals first
-            issue_tile_mma(tmem, a_addr, w_addr, K0, idesc, true);
-            umma::mma_commit(mbar);
-        }
-        const bool ok = __syncthreads_and(umma::mbar_wait(mbar, phase));
-        phase ^= 1u;
-        if (!ok) {
-            flag_timeout(p.err, 1);
-            break;
-        }
-        umma::fence_after_sync();
-        const int64_t m = m0 + row;
-        float x[3] = {0.f, 0.f, 0.f};
-        if (m < q.M) point(m, x);
-        float part4[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll 1
-        for (int c0 = half * 128; c0 < half * 128 + 128; c0 += 32) {
-            float v[32];
-            umma::tmem_ld32(umma::taddr(tmem, qd * 32, c0), v);
-#pragma unroll
-            for (int j = 0; j < 32; ++j) {
-                const int n = c0 + j;
-                const float z = v[j] + w0x_s[3 * n] * x[0] + w0x_s[3 * n + 1] * x[1] + w0x_s[3 * n + 2] * x[2] + b0_s[n];
-                part4[j & 3] = fmaf(wh_s[n], softplus_fast_h(z, spk), part4[j & 3]);
-            }
-        }
-        part_s[half * TILE_M + row] = (part4[0] + part4[1]) + (part4[2] + part4[3]);
-        umma::fence_before_sync();
-        __syncthreads();
-        if (tid < TILE_M && m0 + tid < q.M) q.out[m0 + tid] = q.sign * (part_s[tid] + part_s[TILE_M + tid] + bhead);
-        __syncthreads();
     }
     umma::fence_before_sync();
     __syncthreads();
-    if (warp == 0) umma::tmem_dealloc(tmem, HID);
+    umma::fence_after_sync();
+    const uint32_t tmem = *tslot;
+    const int64_t ntiles = (q.M + TILE_M - 1) / TILE_M;
+
+    if (warp < SP_GATHER_WARPS) {
+        // ---------------- gather ----------------
+        const int row = (warp & 3) * 32 + lane;
+        const __half* const table = (const __half*)p.table;
+        const bool small = q.M <= (int64_t)0xffffffffll;        // 32-bit lattice index arithmetic
+        int it = 0;
+        for (int64_t t = blockIdx.x; t < ntiles; t += gridDim.x, ++it) {
+            const int b = it & 1;
+            if (it >= 2 && !umma::mbar_wait(&done[b], (uint32_t)((it >> 1) - 1) & 1u)) {
+                if (lane == 0) flag_timeout(p.err, 1);
+                break;
+            }
+            const int64_t m = t * TILE_M + row;
+            const bool live = m < q.M;
+            float x[3] = {0.f, 0.f, 0.f};
+            if (live) {
+                if (q.pts) {
+                    x[0] = q.pts[3 * m]; x[1] = q.pts[3 * m + 1]; x[2] = q.pts[3 * m + 2];
+                } else if (small) {
+                    const uint32_t m32 = (uint32_t)m, jk = m32 / (uint32_t)q.nz, i = jk / (uint32_t)q.ny;
+                    x[0] = q.ax[i]; x[1] = q.ay[jk - i * (uint32_t)q.ny]; x[2] = q.az[m32 - jk * (uint32_t)q.nz];
+                } else {
+                    const int64_t jk = m / q.nz, i = jk / q.ny;
+                    x[0] = q.ax[i]; x[1] = q.ay[jk - i * q.ny]; x[2] = q.az[m - jk * q.nz];
+                }
+            }
+            if (warp < 4) {
+                float* xr = x_s + (it & (SP_XRING - 1)) * 3 * TILE_M + row;
+                xr[0] = x[0]; xr[TILE_M] = x[1]; xr[2 * TILE_M] = x[2];
+            }
+            uint8_t* lo_s = a_s + (size_t)(2 * b) * a_bytes;
+            uint8_t* hi_s = lo_s + a_bytes;
+#pragma unroll 1
+            for (int l = warp >> 2; l < A; l += SP_GATHER_WARPS / 4) {
+                uint64_t acc[F / 2];
+#pragma unroll
+                for (int f = 0; f < F / 2; ++f) acc[f] = 0ull;
+                if (live) {
+                    const LevelDesc d = level_desc(p.grid, l);
+                    const GridCell g = grid_cell(d.scale, x);
+                    TableRow<F> r[8];
+#pragma unroll
+                    for (int k = 0; k < 8; ++k)
+                        r[k].load(table + (d.offset + grid_index(d, g.b[0] + (k & 1), g.b[1] + ((k >> 1) & 1),
+                                                                 g.b[2] + ((k >> 2) & 1))) * F);
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) r[k].fma(corner_weight(k, g.f[0], g.f[1], g.f[2]), acc);
+                }
+                float v[F];
+#pragma unroll
+                for (int f = 0; f < F / 2; ++f) unpack_f32x2(acc[f], v[2 * f], v[2 * f + 1]);
+                write_tile_features<F>(hi_s, lo_s, row, l, K0, v);
+            }
+            umma::fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) umma::mbar_arrive(&full[b]);
+        }
+    } else if (warp == SP_GATHER_WARPS + SP_EPI_WARPS) {
+        // ---------------- MMA issue ----------------
+        named_barrier_sync(1, (SP_EPI_WARPS + 1) * 32);          // the weights are staged
+        if (umma::elect_one()) {
+            const uint32_t idesc = umma::idesc_f16(TILE_M, HID);
+            const uint32_t w_addr = umma::smem_u32(w_s), a_addr = umma::smem_u32(a_s);
+            int it = 0;
+            for (int64_t t = blockIdx.x; t < ntiles; t += gridDim.x, ++it) {
+                const int b = it & 1;
+                const uint32_t use = (uint32_t)(it >> 1);
+                if (!umma::mbar_wait(&full[b], use & 1u) || (use > 0 && !umma::mbar_wait(&tempty[b], (use - 1) & 1u))) {
+                    flag_timeout(p.err, 1);
+                    break;
+                }
+                umma::fence_after_sync();
+                const uint32_t d_tmem = tmem + (uint32_t)(b * HID), lo = a_addr + 2u * b * a_bytes;
+                issue_tile_mma(d_tmem, lo, w_addr, K0, idesc);                  // residuals first
+                issue_tile_mma(d_tmem, lo + a_bytes, w_addr, K0, idesc, true);
+                umma::mma_commit(&done[b]);
+                umma::mbar_arrive(&done[b]);         // hands the points' shared-memory writes on, too
+            }
+        }
+        __syncwarp();
+    } else {
+        // ---------------- epilogue ----------------
+        const int et = tid - SP_GATHER_WARPS * 32;
+        stage_rows_kmajor(w_s, (const __half*)p.w0e, 0, HID, K0, K0, et, SP_EPI_WARPS * 32, HID);
+        for (int i = et; i < HID; i += SP_EPI_WARPS * 32) {
+            wx_s[i] = make_float4(p.w0x[3 * i], p.w0x[3 * i + 1], p.w0x[3 * i + 2], p.b0[i]);
+            wh_s[i] = p.whead[i];
+        }
+        cp_async_wait_all();
+        umma::fence_proxy_async_smem();
+        named_barrier_sync(1, (SP_EPI_WARPS + 1) * 32);
+        const float bhead = p.bhead[0];
+        const SoftplusK spk = softplus_k(p.beta);
+        const int qd = warp & 3, half = (warp - SP_GATHER_WARPS) >> 2;
+        const int row = qd * 32 + lane;
+        int it = 0;
+        for (int64_t t = blockIdx.x; t < ntiles; t += gridDim.x, ++it) {
+            const int b = it & 1;
+            // (all eight warps leave together: they share the barriers below)
+            if (!named_barrier_and(2, SP_EPI_WARPS * 32, umma::mbar_wait(&done[b], (uint32_t)(it >> 1) & 1u))) {
+                if (lane == 0) flag_timeout(p.err, 1);
+                break;
+            }
+            umma::fence_after_sync();
+            const float* xr = x_s + (it & (SP_XRING - 1)) * 3 * TILE_M + row;
+            const float x[3] = {xr[0], xr[TILE_M], xr[2 * TILE_M]};
+            float part4[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 1
+            for (int c0 = half * 128; c0 < half * 128 + 128; c0 += 32) {
+                float v[32];
+                umma::tmem_ld32(umma::taddr(tmem, qd * 32, b * HID + c0), v);
+#pragma unroll
+                for (int j = 0; j < 32; ++j) {
+                    const float4 w = wx_s[c0 + j];
+                    const float z = v[j] + w.x * x[0] + w.y * x[1] + w.z * x[2] + w.w;
+                    part4[j & 3] = fmaf(wh_s[c0 + j], softplus_fast_h(z, spk), part4[j & 3]);
+                }
+            }
+            umma::fence_before_sync();
+            __syncwarp();
+            if (lane == 0) umma::mbar_arrive(&tempty[b]);
+            float* ps = part_s + b * 2 * TILE_M;
+            ps[half * TILE_M + row] = (part4[0] + part4[1]) + (part4[2] + part4[3]);
+            named_barrier_sync(2, SP_EPI_WARPS * 32);
+            const int64_t m = t * TILE_M + et;
+            if (et < TILE_M && m < q.M) q.out[m] = q.sign * (ps[et] + ps[TILE_M + et] + bhead);
+        }
+    }
+    umma::fence_before_sync();
+    __syncthreads();
+    if (warp == SP_GATHER_WARPS + SP_EPI_WARPS) umma::tmem_dealloc(tmem, 2 * HID);
 }
 
 static int num_sms() {
@@ -1828,7 +1913,7 @@ extern "C" int gbsdf_sdf_points(const gbsdf_field_args* params, int64_t M, const
         GBSDF_CHECK_ARG(ax && ay && az && nx > 0 && ny > 0 && nz > 0 && (int64_t)nx * ny * nz == M,
                         "lattice mode needs axes with nx*ny*nz == M");
     }
-    const size_t smem = (size_t)HID * p.K0 * 2 + 2 * (size_t)TILE_M * p.K0 * 2 + (HID * 5 + 2 * TILE_M) * 4 + 16;
+    const size_t smem = sdf_points_smem(p.K0);
     GBSDF_CHECK_ARG(smem <= 227 * 1024, "K0 too large");
     const int64_t ntiles = (M + TILE_M - 1) / TILE_M;
     int64_t grid = num_sms();
@@ -1837,15 +1922,15 @@ extern "C" int gbsdf_sdf_points(const gbsdf_field_args* params, int64_t M, const
     switch (p.grid.n_features) {
         case 2:
             allow_max_smem(k_sdf_points<2>);
-            k_sdf_points<2><<<(unsigned)grid, FIELD_THREADS, smem, s>>>(p, q);
+            k_sdf_points<2><<<(unsigned)grid, SP_TPB, smem, s>>>(p, q);
             break;
         case 4:
             allow_max_smem(k_sdf_points<4>);
-            k_sdf_points<4><<<(unsigned)grid, FIELD_THREADS, smem, s>>>(p, q);
+            k_sdf_points<4><<<(unsigned)grid, SP_TPB, smem, s>>>(p, q);
             break;
         default:
             allow_max_smem(k_sdf_points<8>);
-            k_sdf_points<8><<<(unsigned)grid, FIELD_THREADS, smem, s>>>(p, q);
+            k_sdf_points<8><<<(unsigned)grid, SP_TPB, smem, s>>>(p, q);
             break;
     }
     return launch_status("sdf_points");

@@ -95,6 +95,69 @@ def test_gather_rows_match_the_oracle_at_every_evaluation(case):
     assert (got[:, AF:K0] == 0).all() and (got[:, K0 + 16 + AF:] == 0).all()
 
 
+SMS = 152
+# (F, levels, active, points): one point, a tile's edges, one to six tiles per resident CTA, a
+# level count whose columns need padding
+POINTS = [(8, 16, 16, 1), (8, 16, 5, 127), (8, 16, 8, 128), (4, 8, 3, 129), (8, 16, 16, 128 * SMS + 1),
+          (2, 6, 6, 128 * SMS * 2 + 77), (8, 16, 7, 128 * SMS * 5 + 3)]
+
+
+@pytest.mark.parametrize("lattice", [False, True])
+@pytest.mark.parametrize("case", POINTS)
+def test_sdf_points_match_float64_at_tile_edges(case, lattice):
+    F, levels, active, n = case
+    f = Field(F, 6, levels, active, 0.25, 20)
+    g = torch.Generator().manual_seed(n)
+    if lattice:
+        nz = min(n, 13)
+        ny = max(1, min(n // nz, 11))
+        dims = (max(1, n // (nz * ny)), ny, nz)
+        ax = [torch.rand(k, generator=g) * 2 - 1 for k in dims]
+        pts = torch.stack(torch.meshgrid(*ax, indexing="ij"), -1).reshape(-1, 3)
+    else:
+        pts = torch.rand(n, 3, generator=g) * 2 - 1
+    K0, AF, H = f.K0, f.active * F, 256
+    w0e = torch.zeros(H, K0, dtype=torch.float16)
+    w0e[:, :AF] = (torch.randn(H, AF, generator=g) * 0.1).half()
+    w0x, b0 = torch.randn(H, 3, generator=g) * 0.1, torch.randn(H, generator=g) * 0.05
+    wh, bh = torch.randn(H, generator=g) * 0.1, torch.randn(1, generator=g)
+    dev = dict(w0e=w0e, w0x=w0x, b0=b0, whead=wh, bhead=bh)
+    f.keep.update({k: v.to(DEV).contiguous() for k, v in dev.items()})
+    for k in dev:
+        setattr(f.a, k, f.keep[k].data_ptr())
+    f.a.beta = 100.0
+    out = torch.full((len(pts),), float("nan"), device=DEV)
+    err = torch.zeros(1, device=DEV, dtype=torch.int32)
+    f.a.err = err.data_ptr()
+    null = [None] * 4
+    if lattice:
+        axd = [a.to(DEV) for a in ax]
+        where = [None] + [ctypes.c_void_p(a.data_ptr()) for a in axd]
+        shape = dims
+    else:
+        pd = pts.to(DEV)
+        where, shape = [ctypes.c_void_p(pd.data_ptr())] + null[1:], (0, 0, 0)
+    _lib.call("gbsdf_sdf_points", ctypes.byref(f.a), len(pts), *where, *shape, ctypes.c_float(-1.0),
+              ctypes.c_void_p(out.data_ptr()), _lib.stream_ptr(torch.device(DEV)))
+    torch.cuda.synchronize()
+    assert err.item() == 0
+    pick = np.unique(np.concatenate([np.arange(min(len(pts), 300)), np.arange(max(0, len(pts) - 300), len(pts)),
+                                     torch.randint(0, len(pts), (400,), generator=g).numpy()]))
+    p32 = pts.numpy()[pick]
+    enc = hg.encode((p32 + np.float32(2)) * np.float32(0.25), f.table.double().numpy(), f.ora, f.active)[:, :AF]
+    W, X, B = w0e[:, :AF].double().numpy(), w0x.double().numpy(), b0.double().numpy()
+    z = enc @ W.T + p32.astype(np.float64) @ X.T + B
+    h = np.logaddexp(0.0, 100.0 * z) / 100.0
+    a = np.abs(wh.double().numpy())
+    want = -(h @ wh.double().numpy() + bh.double().item())
+    # pre-activation: K0 + 8 float32 roundings of its terms; softplus: 1e-5 relative, 2e-8
+    # absolute; head: 256 roundings of its terms
+    dz = (K0 + 8) * 2.0 ** -22 * (np.abs(enc) @ np.abs(W).T + np.abs(p32) @ np.abs(X).T + np.abs(B))
+    bound = (dz + 1e-5 * h + 2e-8 + 256 * 2.0 ** -24 * h) @ a + 2.0 ** -22
+    assert (np.abs(out.double().cpu().numpy()[pick] - want) <= bound).all()
+    assert torch.isfinite(out).all()
+
+
 @pytest.mark.parametrize("fixed", [False, True])
 @pytest.mark.parametrize("case", CASES)
 def test_scatter_matches_the_oracle_sum_over_evaluations(case, fixed):
