@@ -1434,7 +1434,7 @@ struct SdfPointsArgs {
 //                half of the hidden units per warp; tempty[b] hands the accumulator back.
 // Gather, MMAs and epilogue of one tile used to follow one another in eight warps, so the
 // table's latency stood in every tile.  2.1 M lattice points x 16 levels: 3.79 ms
-// in that form, 1.16 ms in this one; 5.5 M scattered points of a view (four calls) 12.1 and 4.0 ms.
+// in that form, 1.16 ms in this one; 5.5 M scattered points of a view (four calls) 12.1 and 4.4 ms.
 constexpr int SP_GATHER_WARPS = 16;
 constexpr int SP_EPI_WARPS = 8;
 constexpr int SP_TPB = (SP_GATHER_WARPS + SP_EPI_WARPS + 1) * 32;

@@ -16,9 +16,13 @@
 //                      64-column box of X;
 //   warp 1 (one lane)  MMA: per stage, 4 K-steps into the TMEM accumulator [128 x K],
 //                      the lo half first (small addends keep their bits in FP32);
-//   warps 2-5          epilogue once, after the last stage: TMEM -> registers ->
-//                      FP32 atomics into dW (CTAs of other row ranges add into the
-//                      same rows).
+//   warps 2-5          epilogue once, after the last stage: TMEM -> registers -> shared
+//                      memory (the stages are free by then) -> FP32 atomics into dW,
+//                      four columns each and whole rows of 128 bytes per eight lanes (CTAs
+//                      of other row ranges add into the same rows).  Straight from the
+//                      registers, one row per lane, every atomic was a 32-byte sector of
+//                      its own, 5.1 M of them for a 256 x 264 gradient: a step of 512
+//                      rays with 14 such gradients took 2.09 ms that way, 1.73 ms this way.
 // The CTAs of one row range (dW rows 0-127, 128-255, ...) are neighbours in the grid,
 // so the repeated reads of each X box come from L2.
 // Every wait is bounded; a timed-out wait sets *err and the roles leave their loops.
@@ -33,6 +37,7 @@ constexpr int WG_NB = 128;                   // dW rows per CTA (the MMA's M)
 constexpr int WG_THREADS = 192;              // TMA warp, MMA warp, 4 epilogue warps
 constexpr int WG_MAX_STAGES = 4;
 constexpr uint32_t WG_BOX = WG_ROWS * 128;   // one 64-column x 64-row fp16 box: 8 KB
+constexpr int WG_LDS = 36;                   // floats per row of the epilogue's 32 x 32 blocks
 constexpr size_t WG_SMEM_MAX = 227 * 1024;
 constexpr size_t WG_BAR_BYTES = (2 * WG_MAX_STAGES + 2) * 8;
 
@@ -48,6 +53,7 @@ struct WgradParams {
     uint32_t tmem_cols;
     float* dW;
     int ldw;
+    int vec;                // dW's rows are 16-byte aligned: four columns per atomic
     int* err;
 };
 
@@ -157,15 +163,33 @@ __global__ void __launch_bounds__(WG_THREADS, 1) k_wgrad(const __grid_constant__
             if (lane == 0) flag_timeout(p.err, 1);
         } else {
             umma::fence_after_sync();
-            const int n = n0 + q * 32 + lane;
-            float* dst = p.dW + (int64_t)n * p.ldw;
+            // this warp's 32 x 32 block, rows padded to keep both directions free of conflicts
+            float* blk = reinterpret_cast<float*>(smem) + q * (32 * WG_LDS);
+            const int r4 = lane >> 3, j4 = (lane & 7) * 4;
             for (int c = 0; c < p.K; c += 32) {
                 float v[32];
                 umma::tmem_ld32(umma::taddr(tmem, q * 32, (uint32_t)c), v);
-                if (n < p.N) {
+                __syncwarp();                        // the previous block has been read
 #pragma unroll
-                    for (int j = 0; j < 32; ++j)
-                        if (c + j < p.K && v[j] != 0.0f) atomicAdd(dst + c + j, v[j]);
+                for (int j = 0; j < 32; j += 4)
+                    *reinterpret_cast<float4*>(blk + lane * WG_LDS + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+                __syncwarp();
+                const int left = p.K - c - j4;       // columns of dW from this lane's first one on
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const int r = 4 * i + r4, n = n0 + q * 32 + r;
+                    if (n >= p.N || left <= 0) continue;
+                    const float4 a = *reinterpret_cast<const float4*>(blk + r * WG_LDS + j4);
+                    float* dst = p.dW + (int64_t)n * p.ldw + c + j4;
+                    if (p.vec && left >= 4) {
+                        if (a.x != 0.0f || a.y != 0.0f || a.z != 0.0f || a.w != 0.0f)
+                            atomicAdd(reinterpret_cast<float4*>(dst), a);
+                    } else {
+                        if (a.x != 0.0f) atomicAdd(dst, a.x);
+                        if (left > 1 && a.y != 0.0f) atomicAdd(dst + 1, a.y);
+                        if (left > 2 && a.z != 0.0f) atomicAdd(dst + 2, a.z);
+                        if (left > 3 && a.w != 0.0f) atomicAdd(dst + 3, a.w);
+                    }
                 }
             }
         }
@@ -233,6 +257,7 @@ extern "C" int gbsdf_wgrad(int64_t M, int N, int K, const void* dZ, const void* 
     p.rows_per_cta = (stages + splits - 1) / splits * WG_ROWS;
     splits = (M + p.rows_per_cta - 1) / p.rows_per_cta;
     p.dW = dW; p.ldw = ldw; p.err = err;
+    p.vec = aligned(dW, 16) && ldw % 4 == 0 ? 1 : 0;
     CUtensorMap tm_z, tm_zlo, tm_x;
     const CUtensorMapL2promotion l2 = CU_TENSOR_MAP_L2_PROMOTION_L2_256B;
     if (int st = tensor_map_2d(&tm_z, false, dZ, M, N, ldz, 64, WG_ROWS, CU_TENSOR_MAP_SWIZZLE_128B, l2, "dZ"))

@@ -70,3 +70,19 @@ def test_wgrad_rejects_bad_arguments():
     dW = torch.zeros(1024, 64, device=DEV)
     with pytest.raises(RuntimeError, match="at most 512"):
         fused._wgrad(dZ, X, 1024, 64, dW)
+
+
+@pytest.mark.parametrize("N,K,ld,shift", [(200, 33, 41, 0), (200, 34, 36, 0), (128, 264, 264, 1), (1, 3, 4, 0)])
+def test_wgrad_columns_that_do_not_fill_a_vector(N, K, ld, shift):
+    """Columns left over after the four-column atomics, rows and bases that are not 16-byte
+    aligned: FP32 sums of M exact products, at most 2 M roundings of the sum of magnitudes."""
+    M = 700
+    g = torch.Generator(DEV).manual_seed(N + K)
+    dZ = torch.randn(M, (N + 7) // 8 * 8, device=DEV, generator=g).half()
+    X = torch.randn(M, (K + 7) // 8 * 8, device=DEV, generator=g).half()
+    flat = torch.full((shift + N * ld + 8,), 5.0, device=DEV)
+    dW = flat[shift:shift + N * ld].view(N, ld)
+    fused._wgrad(dZ, X, N, K, dW[:, :K])
+    bound = 2 * M * 2.0 ** -24 * ref(dZ.abs(), X.abs(), N, K)
+    assert bool(((dW[:, :K].double() - ref(dZ, X, N, K)).abs() <= bound).all())
+    assert bool((dW[:, K:] == 5.0).all()) and bool((flat[:shift] == 5.0).all())
