@@ -567,7 +567,6 @@ __global__ void __launch_bounds__(SCATTER_THREADS, CPT >= 8 ? 2 : (CPT == 4 ? 3 
 // bias columns], so the epilogue reads W0x x + b0 + W0e f from TMEM and adds
 // nothing; the fp16 residual of the features is a second MMA over the W0e prefix.
 constexpr int FWD_CTAS_PER_SM = 2;
-constexpr int FWD_APP_MAX = 28;        // appearance-code columns the forward's prefetch holds
 // One sample's per-ray inputs of the forward's per-sample phase, prefetched into a ring of
 // four tiles in shared memory (see k_field_fwd)
 struct FwdSample {
@@ -576,50 +575,72 @@ struct FwdSample {
     int appi;                    // appearance-code row
     float c[3];                  // sample point c + d t
     float dv[3];                 // ray direction
-    float app[FWD_APP_MAX];      // appearance code
 };
 constexpr int FWD_RING = 4;
-// the colour-input tail is at most 48 columns with 23 fixed ones (check_fwd): app_dim <= 25
-static_assert(FWD_APP_MAX >= 48 - 23, "the prefetch record holds every appearance column");
+constexpr int FWD_APP_RING = 2;  // appearance codes: this tile's and the next one's
 
-template <int F, int TAPS>
-__global__ void __launch_bounds__(FIELD_THREADS, FWD_CTAS_PER_SM) k_field_fwd(FieldParams p,
-                                                                             const __grid_constant__ CUtensorMap tm_xhi,
-                                                                             const __grid_constant__ CUtensorMap tm_xlo) {
+// shared memory of one group: feature tiles, partial sums, SDF values, barriers, prefetch rings
+// (16-byte multiples, so that every group's feature tile stays aligned)
+// (appearance rows an odd number of floats apart: one bank each)
+__host__ __device__ constexpr int fwd_app_ld(int app_dim) { return app_dim > 0 ? app_dim | 1 : 0; }
+template <int TAPS>
+__host__ __device__ constexpr int fwd_group_bytes(int K0, int app_dim) {
+    return (TILE_M * (2 * K0 + 16) * 2 + (2 * TILE_M + FWD_SDF_FLOATS) * 4 + 24 +
+            FWD_RING * TapTile<TAPS>::SPT * (int)sizeof(FwdSample) +
+            FWD_APP_RING * TapTile<TAPS>::SPT * fwd_app_ld(app_dim) * 4 + 127) / 128 * 128;
+}
+
+// GROUPS: independent groups of eight warps in a CTA, each on tiles of its own with its own
+// feature buffers, accumulator and barriers, sharing the resident weights.  Where the shared
+// memory holds two CTAs per SM (K0 <= 80) one group per CTA is the same thing; above that one
+// CTA of two groups keeps two tiles in flight per SM where one CTA of one group left every
+// phase exposed.  K0 = 128 (16 levels x 8 features): 6.3 M samples 15.4 ms with one group, 12.7
+// with two; 0.24 M samples 0.50 and 0.40 ms.
+template <int F, int TAPS, int GROUPS>
+__global__ void __launch_bounds__(FIELD_THREADS * GROUPS, GROUPS == 1 ? FWD_CTAS_PER_SM : 1)
+    k_field_fwd(FieldParams p, const __grid_constant__ CUtensorMap tm_xhi, const __grid_constant__ CUtensorMap tm_xlo) {
     constexpr int EVALS = TapTile<TAPS>::EVALS, SPT = TapTile<TAPS>::SPT;
     extern __shared__ __align__(1024) uint8_t smem[];
     const int K0 = p.K0;
     const int KB = K0 + 16;                                     // features hi + tail
     const int KX = 2 * K0 + 16;                                 // x0ext row width
+    const int grp = GROUPS == 1 ? 0 : (int)(threadIdx.x / FIELD_THREADS);
+    const int app_cols = p.xc ? p.app_dim : 0, app_ld = fwd_app_ld(app_cols), group_bytes = fwd_group_bytes<TAPS>(K0, app_cols);
     uint8_t* w_s = smem;                                        // [256 x KB]  w0b
-    uint8_t* a_s = w_s + HID * KB * 2;                          // [128 x KB]  features hi | tail
+    float* wh_s = reinterpret_cast<float*>(w_s + HID * KB * 2); // [256]
+    uint8_t* a_s = reinterpret_cast<uint8_t*>(wh_s + HID) + grp * group_bytes;   // [128 x KB]  features hi | tail
     uint8_t* a2_s = a_s + TILE_M * KB * 2;                      // [128 x K0]  features lo
-    float* wh_s = reinterpret_cast<float*>(a2_s + TILE_M * K0 * 2);   // [256]
-    float* part_s = wh_s + HID;                                 // [2][128] partial head sums
+    float* part_s = reinterpret_cast<float*>(a2_s + TILE_M * K0 * 2);   // [2][128] partial head sums
     float* sdf_s = part_s + 2 * TILE_M;                         // [7][18]
     // the mbarrier 8-byte aligned whatever the tile's row count: 128 floats past sdf_s
     // (125 or 126 evaluation rows + padding)
     uint64_t* mbar = reinterpret_cast<uint64_t*>(sdf_s + FWD_SDF_FLOATS);
     uint64_t* mbar_a = mbar + 1;                                // the A tile's TMA loads
-    uint32_t* tslot = reinterpret_cast<uint32_t*>(mbar + 2);
-    FwdSample* ring = reinterpret_cast<FwdSample*>(mbar + 3);  // [FWD_RING][SPT]
+    uint32_t* tslot = reinterpret_cast<uint32_t*>(mbar + 2);    // (group 0's)
+    FwdSample* ring = reinterpret_cast<FwdSample*>(mbar + 3);   // [FWD_RING][SPT]
+    float* app_s = reinterpret_cast<float*>(ring + FWD_RING * SPT);   // [FWD_APP_RING][SPT][app_ld]
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    stage_rows_kmajor(w_s, (const __half*)p.w0b, 0, HID, KB, KB, tid, FIELD_THREADS, HID);
-    for (int i = tid; i < HID; i += FIELD_THREADS) wh_s[i] = p.whead[i];
+    // thread and warp within the group; the group's barrier
+    const int tid = threadIdx.x % FIELD_THREADS, warp = tid >> 5, lane = tid & 31;
+    auto group_sync = [&]() { named_barrier_sync(1 + grp, FIELD_THREADS); };
+    stage_rows_kmajor(w_s, (const __half*)p.w0b, 0, HID, KB, KB, threadIdx.x, FIELD_THREADS * GROUPS, HID);
+    for (int i = threadIdx.x; i < HID; i += FIELD_THREADS * GROUPS) wh_s[i] = p.whead[i];
     if (tid == 0) {
         umma::mbar_init(mbar, 1);
         umma::mbar_init(mbar_a, 1);
         umma::fence_mbar_init();
     }
-    if (warp == 0) {
-        umma::tmem_alloc(tslot, HID);
+    if (threadIdx.x < 32) {
+        umma::tmem_alloc(tslot, HID * GROUPS);
         umma::tmem_relinquish();
     }
     cp_async_wait_all();
+    umma::fence_proxy_async_smem();
+    umma::fence_before_sync();
     __syncthreads();
     umma::fence_after_sync();
-    const uint32_t tmem = *tslot;
+    const uint32_t tmem0 = *reinterpret_cast<uint32_t*>(reinterpret_cast<uint8_t*>(tslot) - grp * group_bytes);
+    const uint32_t tmem = tmem0 + (uint32_t)(grp * HID);
     const uint32_t idesc = umma::idesc_f16(TILE_M, HID);
     const uint32_t a_addr = umma::smem_u32(a_s), w_addr = umma::smem_u32(w_s), a2_addr = umma::smem_u32(a2_s);
     const float bhead = p.bhead[0];
@@ -664,7 +685,8 @@ __global__ void __launch_bounds__(FIELD_THREADS, FWD_CTAS_PER_SM) k_field_fwd(Fi
     const bool want_xc = p.xc != nullptr;
     const bool want_app = want_xc && p.app_table && p.app_dim > 0;
     auto slot = [&](int k) { return ring + (k & (FWD_RING - 1)) * SPT; };
-    auto tile_of = [&](int k) { return (int64_t)blockIdx.x + (int64_t)k * gridDim.x; };
+    auto app_of = [&](int k, int js) { return app_s + ((k & (FWD_APP_RING - 1)) * SPT + js) * app_ld; };
+    auto tile_of = [&](int k) { return (int64_t)blockIdx.x * GROUPS + grp + (int64_t)k * gridDim.x * GROUPS; };
     auto pre_ray = [&](int k, int js) {
         const int64_t tk = tile_of(k), ss = tk * SPT + js;
         slot(k)[js].r = (tk < ntiles && ss < p.Ns) ? ray_of(p, ss) : -1;
@@ -683,8 +705,9 @@ __global__ void __launch_bounds__(FIELD_THREADS, FWD_CTAS_PER_SM) k_field_fwd(Fi
         if (want_app) e.appi = p.app_idx[r];
     };
     auto pre_app = [&](int k, int js) {
-        FwdSample& e = slot(k)[js];
+        const FwdSample& e = slot(k)[js];
         if (e.r < 0 || !want_app) return;
+        float* dst = app_of(k, js);
         const float* a = p.app_table + (int64_t)e.appi * p.app_dim;
         for (int i0 = 0; i0 < p.app_dim; i0 += 8) {
             float v[8];
@@ -692,7 +715,7 @@ __global__ void __launch_bounds__(FIELD_THREADS, FWD_CTAS_PER_SM) k_field_fwd(Fi
             for (int j = 0; j < 8; ++j) v[j] = i0 + j < p.app_dim ? a[i0 + j] : 0.0f;
 #pragma unroll
             for (int j = 0; j < 8; ++j)
-                if (i0 + j < p.app_dim) e.app[i0 + j] = v[j];
+                if (i0 + j < p.app_dim) dst[i0 + j] = v[j];
         }
     };
     constexpr int LD0 = (SPT * 6 + 31) / 32 * 32;    // first loader thread
@@ -702,27 +725,28 @@ __global__ void __launch_bounds__(FIELD_THREADS, FWD_CTAS_PER_SM) k_field_fwd(Fi
         pre_ray(1, tid);
         pre_ray(2, tid);
     }
-    __syncthreads();
+    group_sync();
     if (tid < SPT) {
         pre_vals(0, tid);
         pre_vals(1, tid);
     }
-    __syncthreads();
+    group_sync();
     if (tid < SPT) pre_app(0, tid);
-    int64_t t = blockIdx.x;
+    int64_t t = tile_of(0);
+    const int64_t t_step = (int64_t)gridDim.x * GROUPS;
     if (t < ntiles && tid == 0) load_a(t);
-    __syncthreads();
+    group_sync();
     if (t < ntiles) issue(0u);
-    for (int it = 0; t < ntiles; t += gridDim.x, ++it) {
+    for (int it = 0; t < ntiles; t += t_step, ++it) {
         const int64_t s0 = t * SPT;
-        const bool ok = __syncthreads_and(umma::mbar_wait(mbar, phase));
+        const bool ok = named_barrier_and(1 + grp, FIELD_THREADS, umma::mbar_wait(mbar, phase));
         phase ^= 1u;
         if (!ok) {
             flag_timeout(p.err, 1);
             break;
         }
         umma::fence_after_sync();
-        const int64_t tn = t + gridDim.x;
+        const int64_t tn = t + t_step;
         if (tn < ntiles && tid == 0) load_a(tn);
         // epilogue: h = softplus(pre) ; partial head dot ; centre rows keep h in h0c
         const int64_t s = s0 + sl_row;
@@ -753,11 +777,11 @@ __global__ void __launch_bounds__(FIELD_THREADS, FWD_CTAS_PER_SM) k_field_fwd(Fi
         }
         part_s[half * TILE_M + row] = (part4[0] + part4[1]) + (part4[2] + part4[3]);
         umma::fence_before_sync();
-        __syncthreads();
+        group_sync();
         if (tid < SPT * EVALS) {
             sdf_s[tid] = part_s[tid] + part_s[TILE_M + tid] + bhead;
         }
-        __syncthreads();
+        group_sync();
         // per-sample: gradient, Hessian diagonal, outside overwrite, colour-input columns;
         // six threads per sample, each storing one 8-column chunk of the colour-input tail
         // (the first of them also the SDF, gradient and Hessian)
@@ -837,7 +861,7 @@ __global__ void __launch_bounds__(FIELD_THREADS, FWD_CTAS_PER_SM) k_field_fwd(Fi
                     // compile-time indices (col[] stays in registers), the appearance code read
                     // straight from the table, and the last (padding) column a constant 1: the
                     // colour layer-0 weight gradient dZ^T xc then carries the bias gradient there
-                    const float* a = want_app ? e.app : nullptr;
+                    const float* a = want_app ? app_of(it, js) : nullptr;
                     (void)r;
                     __half* dst = (__half*)p.xc + ss * (int64_t)p.ldxc + HID;
                     const int ncol = p.ldxc - HID;
@@ -858,12 +882,12 @@ __global__ void __launch_bounds__(FIELD_THREADS, FWD_CTAS_PER_SM) k_field_fwd(Fi
                 }
             }
         }
-        __syncthreads();
+        group_sync();
         if (tn < ntiles) issue((uint32_t)(it + 1) & 1u);
     }
     umma::fence_before_sync();
     __syncthreads();
-    if (warp == 0) umma::tmem_dealloc(tmem, HID);
+    if (threadIdx.x < 32) umma::tmem_dealloc(tmem0, HID * GROUPS);
 }
 
 // ---------------------------------------------------------------------------
@@ -1624,11 +1648,8 @@ static int num_sms() {
 }
 
 template <int TAPS>
-static size_t fwd_smem(int K0) {
-    const size_t KB = (size_t)K0 + 16;
-    return (size_t)HID * KB * 2 + (size_t)TILE_M * (KB + K0) * 2 +
-           (HID + 2 * TILE_M + FWD_SDF_FLOATS) * 4 + 24 +
-           (size_t)FWD_RING * TapTile<TAPS>::SPT * sizeof(FwdSample);
+static size_t fwd_smem(int K0, int app_dim, int groups) {
+    return (size_t)HID * (K0 + 16) * 2 + HID * 4 + (size_t)groups * fwd_group_bytes<TAPS>(K0, app_dim);
 }
 template <int TAPS>
 static size_t bwd_smem(int K0, bool dw) {
@@ -1675,18 +1696,31 @@ static int launch_field(const FieldParams& p, int which, cudaStream_t s) {
         if (int st = launch_status("field gather")) return st;
     }
     if (which & FK_MLP_FWD) {
-        const size_t smem = fwd_smem<TAPS>(p.K0);
-        if (smem > 227 * 1024) {
-            set_error("field forward needs %zu B of shared memory", smem);
+        constexpr size_t limit = 227 * 1024, per_sm = 228 * 1024, reserved = 1024;   // per CTA, per SM, per CTA resident
+        const int app_cols = p.xc ? p.app_dim : 0;
+        const size_t one = fwd_smem<TAPS>(p.K0, app_cols, 1);
+        if (one > limit) {
+            set_error("field forward needs %zu B of shared memory", one);
             return GBSDF_ERR_UNSUPPORTED;
         }
-        // p.fwd_ctas (a tuning choice): resident CTAs per SM to launch, 1 or 2 (0 = 2)
-        int64_t grid = num_sms() * (p.fwd_ctas == 1 ? 1 : FWD_CTAS_PER_SM);
-        if (grid > ntiles) grid = ntiles;
+        // Two tiles in flight per SM: two CTAs where they fit, else (K0 > 80) one CTA of two groups
+        // where that fits (with 4 taps' larger rings not K0 = 128 and more than 17 appearance columns).
+        // p.fwd_ctas (a tuning choice): 1 keeps one tile in flight (0 = 2)
+        const bool two = p.fwd_ctas != 1;
+        const int groups = two && FWD_CTAS_PER_SM * (one + reserved) > per_sm && fwd_smem<TAPS>(p.K0, app_cols, 2) <= limit ? 2 : 1;
+        const size_t smem = fwd_smem<TAPS>(p.K0, app_cols, groups);
+        int64_t grid = num_sms() * (two && groups == 1 ? FWD_CTAS_PER_SM : 1);
+        const int64_t need = (ntiles + groups - 1) / groups;
+        if (grid > need) grid = need;
         CUtensorMap tm_xhi, tm_xlo;
         if (int st = x0ext_maps(p, ntiles * TILE_ROWS, p.K0, &tm_xhi, &tm_xlo)) return st;
-        allow_max_smem(k_field_fwd<F, TAPS>);
-        k_field_fwd<F, TAPS><<<(unsigned)grid, FIELD_THREADS, smem, s>>>(p, tm_xhi, tm_xlo);
+        if (groups == 2) {
+            allow_max_smem(k_field_fwd<F, TAPS, 2>);
+            k_field_fwd<F, TAPS, 2><<<(unsigned)grid, 2 * FIELD_THREADS, smem, s>>>(p, tm_xhi, tm_xlo);
+        } else {
+            allow_max_smem(k_field_fwd<F, TAPS, 1>);
+            k_field_fwd<F, TAPS, 1><<<(unsigned)grid, FIELD_THREADS, smem, s>>>(p, tm_xhi, tm_xlo);
+        }
         if (int st = launch_status("field forward")) return st;
     }
     if (which & FK_MLP_BWD) {

@@ -158,6 +158,47 @@ def test_sdf_points_match_float64_at_tile_edges(case, lattice):
     assert torch.isfinite(out).all()
 
 
+# (taps, active levels of 8 features, appearance columns, samples): K0 = 96..128, where two tiles
+# share a CTA; one tile, two, an odd number, more than two per CTA, a ragged last one
+FORWARD = [(6, 16, 16, 1), (6, 16, 16, 36), (6, 12, 25, 50), (4, 16, 16, 60), (4, 16, 25, 26), (6, 14, 0, 18 * SMS * 3 + 5),
+           (4, 13, 16, 25 * SMS * 5 + 1)]
+
+
+@pytest.mark.parametrize("case", FORWARD)
+def test_forward_with_two_tiles_per_cta_equals_one(case):
+    """fwd_ctas = 1 keeps one tile in flight; the outputs do not depend on it, bit for bit."""
+    taps, active, app, n = case
+    f = Field(8, taps, 16, active, 0.25, n)
+    g = torch.Generator().manual_seed(n)
+    r = lambda *s: torch.randn(*s, generator=g)  # noqa: E731
+    f.a.beta, f.a.two_eps, f.a.eps2, f.a.outside_val = 100.0, 2 * f.a.eps, f.a.eps ** 2, 1000.0
+    ldxc = 256 + (22 + app + 1 + 15) // 16 * 16
+    dev = dict(w0b=(r(256, f.K0 + 16) * 0.1).half(), whead=r(256) * 0.1, bhead=r(1), app_table=r(4, max(app, 1)),
+               app_idx=torch.tensor([2, 0, 3], dtype=torch.int32), outside=torch.tensor([0, 1, 0], dtype=torch.uint8))
+    f.keep.update({k: v.to(DEV) for k, v in dev.items()})
+    for k in dev:
+        setattr(f.a, k, f.keep[k].data_ptr())
+    f.a.app_dim, f.a.ldxc, f.a.ld_h0c = app, ldxc, 256
+    x0 = torch.zeros(f.rows, 2 * f.K0 + 16, device=DEV, dtype=torch.float16)
+    err = torch.zeros(1, device=DEV, dtype=torch.int32)
+    f.a.x0ext, f.a.err = x0.data_ptr(), err.data_ptr()
+    f.call("gbsdf_field_encode")
+    got = []
+    for ctas in (1, 2):
+        h = lambda w: torch.full((n, w), -7.0, device=DEV, dtype=torch.float16)  # noqa: E731
+        o = dict(sdf=torch.full((n,), -7.0, device=DEV), grad=torch.full((n, 3), -7.0, device=DEV),
+                 hess=torch.full((n, 3), -7.0, device=DEV), h0c=h(256), h0c_lo=h(256), xc=h(ldxc), xc_lo=h(ldxc))
+        for k, v in o.items():
+            setattr(f.a, k, v.data_ptr())
+        f.a.fwd_ctas = ctas
+        f.call("gbsdf_field_mlp_fwd")
+        got.append(o)
+    assert err.item() == 0
+    for k in got[0]:
+        assert torch.equal(got[0][k], got[1][k]), k
+    assert bool((got[1]["xc"][:, :256] == -7).all()) and bool((got[1]["sdf"] != -7).all())
+
+
 @pytest.mark.parametrize("fixed", [False, True])
 @pytest.mark.parametrize("case", CASES)
 def test_scatter_matches_the_oracle_sum_over_evaluations(case, fixed):
