@@ -580,14 +580,22 @@ constexpr int FWD_RING = 4;
 constexpr int FWD_APP_RING = 2;  // appearance codes: this tile's and the next one's
 
 // shared memory of one group: feature tiles, partial sums, SDF values, barriers, prefetch rings
-// (16-byte multiples, so that every group's feature tile stays aligned)
+// (1024-byte multiples, as the swizzled feature tiles need)
+//
+// The feature tiles: 64-column boxes of 128 rows in the 128-byte swizzle, ceil(K0 / 64) of the
+// hi columns (from column 0) and of the lo columns (from K0 + 16), and the 16 tail columns as two
+// 16-byte chunks of 128 rows without a swizzle.  A box row is a 128-byte line; the core-matrix
+// layout, loaded as 16-byte rows, moved 8 times as many of them and bounded the kernel: 12.7 ms
+// for 6.3 M samples at K0 = 128 against 9.8, 2.80 ms for 2.1 M at K0 = 64 against 2.38.
+constexpr int FWD_BOX_BYTES = TILE_M * 128;
+__host__ __device__ constexpr int fwd_tile_bytes(int K0) { return 2 * ((K0 + 63) / 64) * FWD_BOX_BYTES + TILE_M * 32; }
 // (appearance rows an odd number of floats apart: one bank each)
 __host__ __device__ constexpr int fwd_app_ld(int app_dim) { return app_dim > 0 ? app_dim | 1 : 0; }
 template <int TAPS>
 __host__ __device__ constexpr int fwd_group_bytes(int K0, int app_dim) {
-    return (TILE_M * (2 * K0 + 16) * 2 + (2 * TILE_M + FWD_SDF_FLOATS) * 4 + 24 +
+    return (fwd_tile_bytes(K0) + (2 * TILE_M + FWD_SDF_FLOATS) * 4 + 24 +
             FWD_RING * TapTile<TAPS>::SPT * (int)sizeof(FwdSample) +
-            FWD_APP_RING * TapTile<TAPS>::SPT * fwd_app_ld(app_dim) * 4 + 127) / 128 * 128;
+            FWD_APP_RING * TapTile<TAPS>::SPT * fwd_app_ld(app_dim) * 4 + 1023) / 1024 * 1024;
 }
 
 // GROUPS: independent groups of eight warps in a CTA, each on tiles of its own with its own
@@ -595,22 +603,23 @@ __host__ __device__ constexpr int fwd_group_bytes(int K0, int app_dim) {
 // memory holds two CTAs per SM (K0 <= 80) one group per CTA is the same thing; above that one
 // CTA of two groups keeps two tiles in flight per SM where one CTA of one group left every
 // phase exposed.  K0 = 128 (16 levels x 8 features): 6.3 M samples 15.4 ms with one group, 12.7
-// with two; 0.24 M samples 0.50 and 0.40 ms.
+// with two; 0.24 M samples 0.50 and 0.40 ms (both before the swizzled feature tiles).
 template <int F, int TAPS, int GROUPS>
 __global__ void __launch_bounds__(FIELD_THREADS * GROUPS, GROUPS == 1 ? FWD_CTAS_PER_SM : 1)
-    k_field_fwd(FieldParams p, const __grid_constant__ CUtensorMap tm_xhi, const __grid_constant__ CUtensorMap tm_xlo) {
+    k_field_fwd(FieldParams p, const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_tail) {
     constexpr int EVALS = TapTile<TAPS>::EVALS, SPT = TapTile<TAPS>::SPT;
     extern __shared__ __align__(1024) uint8_t smem[];
     const int K0 = p.K0;
     const int KB = K0 + 16;                                     // features hi + tail
-    const int KX = 2 * K0 + 16;                                 // x0ext row width
+    const int nbox = (K0 + 63) / 64;                            // 64-column boxes of the hi (and of the lo) features
     const int grp = GROUPS == 1 ? 0 : (int)(threadIdx.x / FIELD_THREADS);
     const int app_cols = p.xc ? p.app_dim : 0, app_ld = fwd_app_ld(app_cols), group_bytes = fwd_group_bytes<TAPS>(K0, app_cols);
     uint8_t* w_s = smem;                                        // [256 x KB]  w0b
     float* wh_s = reinterpret_cast<float*>(w_s + HID * KB * 2); // [256]
-    uint8_t* a_s = reinterpret_cast<uint8_t*>(wh_s + HID) + grp * group_bytes;   // [128 x KB]  features hi | tail
-    uint8_t* a2_s = a_s + TILE_M * KB * 2;                      // [128 x K0]  features lo
-    float* part_s = reinterpret_cast<float*>(a2_s + TILE_M * K0 * 2);   // [2][128] partial head sums
+    uint8_t* a_s = reinterpret_cast<uint8_t*>(wh_s + HID) + grp * group_bytes;   // [boxes]  features hi
+    uint8_t* a2_s = a_s + nbox * FWD_BOX_BYTES;                 // [boxes]  features lo
+    uint8_t* at_s = a2_s + nbox * FWD_BOX_BYTES;                // [2 chunks][128 x 16 bytes]  tail
+    float* part_s = reinterpret_cast<float*>(at_s + TILE_M * 32);   // [2][128] partial head sums
     float* sdf_s = part_s + 2 * TILE_M;                         // [7][18]
     // the mbarrier 8-byte aligned whatever the tile's row count: 128 floats past sdf_s
     // (125 or 126 evaluation rows + padding)
@@ -643,6 +652,7 @@ __global__ void __launch_bounds__(FIELD_THREADS * GROUPS, GROUPS == 1 ? FWD_CTAS
     const uint32_t tmem = tmem0 + (uint32_t)(grp * HID);
     const uint32_t idesc = umma::idesc_f16(TILE_M, HID);
     const uint32_t a_addr = umma::smem_u32(a_s), w_addr = umma::smem_u32(w_s), a2_addr = umma::smem_u32(a2_s);
+    const uint32_t at_addr = umma::smem_u32(at_s);
     const float bhead = p.bhead[0];
     const int64_t ntiles = (p.Ns + SPT - 1) / SPT;
     const int q = warp & 3, half = warp >> 2;
@@ -650,20 +660,18 @@ __global__ void __launch_bounds__(FIELD_THREADS * GROUPS, GROUPS == 1 ? FWD_CTAS
     const int e_row = row / SPT, sl_row = row % SPT;
     uint32_t phase = 0;
 
-    // features of a tile, gathered by k_field_gather into x0ext, loaded by TMA (thread 0, one
-    // box per 8-row group and part, straight into the core-matrix layout; rows past the end
-    // arrive as zeros); the next tile's load overlaps this tile's epilogue (A is free once its
-    // MMAs completed)
+    // features of a tile, gathered by k_field_gather into x0ext, loaded by TMA (thread 0; rows past
+    // the end arrive as zeros, columns past a part are not used); the next tile's load overlaps
+    // this tile's epilogue (A is free once its MMAs completed)
     // (a timed-out tile ends the loop at its top, before its load_a: no load is left in flight)
-    (void)KX;
     auto load_a = [&](int64_t tt) {
-        umma::mbar_arrive_expect_tx(mbar_a, (uint32_t)(TILE_M * (KB + K0) * 2));
+        umma::mbar_arrive_expect_tx(mbar_a, (uint32_t)fwd_tile_bytes(K0));
         const int row0 = (int)(tt * (SPT * EVALS));
-#pragma unroll 1
-        for (int g = 0; g < TILE_M / 8; ++g) {
-            umma::tma_load_3d(a_s + g * KB * 16, &tm_xhi, 0, row0 + 8 * g, 0, mbar_a);
-            umma::tma_load_3d(a2_s + g * K0 * 16, &tm_xlo, 0, row0 + 8 * g, 0, mbar_a);
+        for (int j = 0; j < nbox; ++j) {
+            umma::tma_load_2d(a2_s + j * FWD_BOX_BYTES, &tm_x, KB + 64 * j, row0, mbar_a);
+            umma::tma_load_2d(a_s + j * FWD_BOX_BYTES, &tm_x, 64 * j, row0, mbar_a);
         }
+        umma::tma_load_3d(at_s, &tm_tail, 0, row0, 0, mbar_a);
     };
     auto issue = [&](uint32_t phase_a) {           // the k-th call waits for the k-th load: phase k & 1
         if (tid == 0) {
@@ -672,8 +680,15 @@ __global__ void __launch_bounds__(FIELD_THREADS * GROUPS, GROUPS == 1 ? FWD_CTAS
             // smallest terms first: the tensor core's FP32 accumulation drops low
             // bits of addends much smaller than the running sum, so the fp16
             // residuals go in before the hi features and the large position/bias tail
-            issue_tile_mma_strided(tmem, a2_addr, K0, w_addr, KB, K0, idesc);
-            issue_tile_mma(tmem, a_addr, w_addr, KB, idesc, true);
+            const uint32_t sbo = (uint32_t)KB * 16u;
+            for (int i = 0; i < 2; ++i) {
+                const uint32_t base = i == 0 ? a2_addr : a_addr;
+                for (int ks = 0; ks < K0 / 16; ++ks)
+                    umma::mma_f16(tmem, umma::make_desc_sw128(base + (ks >> 2) * FWD_BOX_BYTES + (ks & 3) * 32u),
+                                  umma::make_desc(w_addr + ks * 256u, 128u, sbo), idesc, (i > 0 || ks > 0) ? 1u : 0u);
+            }
+            umma::mma_f16(tmem, umma::make_desc(at_addr, TILE_M * 16u, 128u),
+                          umma::make_desc(w_addr + (K0 / 16) * 256u, 128u, sbo), idesc, 1u);
             umma::mma_commit(mbar);
         }
     };
@@ -1712,14 +1727,20 @@ static int launch_field(const FieldParams& p, int which, cudaStream_t s) {
         int64_t grid = num_sms() * (two && groups == 1 ? FWD_CTAS_PER_SM : 1);
         const int64_t need = (ntiles + groups - 1) / groups;
         if (grid > need) grid = need;
-        CUtensorMap tm_xhi, tm_xlo;
-        if (int st = x0ext_maps(p, ntiles * TILE_ROWS, p.K0, &tm_xhi, &tm_xlo)) return st;
+        const int KX = 2 * p.K0 + 16;
+        CUtensorMap tm_x, tm_tail;
+        if (int st = tensor_map_2d(&tm_x, false, p.x0ext, ntiles * TILE_ROWS, KX, KX, 64, TILE_M,
+                                   CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, "x0ext"))
+            return st;
+        if (int st = tensor_map_kmajor_groups(&tm_tail, (const __half*)p.x0ext + p.K0, ntiles * TILE_ROWS, 2, KX, 2,
+                                              "x0ext tail", TILE_M))
+            return st;
         if (groups == 2) {
             allow_max_smem(k_field_fwd<F, TAPS, 2>);
-            k_field_fwd<F, TAPS, 2><<<(unsigned)grid, 2 * FIELD_THREADS, smem, s>>>(p, tm_xhi, tm_xlo);
+            k_field_fwd<F, TAPS, 2><<<(unsigned)grid, 2 * FIELD_THREADS, smem, s>>>(p, tm_x, tm_tail);
         } else {
             allow_max_smem(k_field_fwd<F, TAPS, 1>);
-            k_field_fwd<F, TAPS, 1><<<(unsigned)grid, FIELD_THREADS, smem, s>>>(p, tm_xhi, tm_xlo);
+            k_field_fwd<F, TAPS, 1><<<(unsigned)grid, FIELD_THREADS, smem, s>>>(p, tm_x, tm_tail);
         }
         if (int st = launch_status("field forward")) return st;
     }

@@ -55,8 +55,10 @@ inline int tensor_map_2d(CUtensorMap* map, bool f32, const void* base, int64_t r
 // row, chunk) with strides (row pitch, 16 B), so a box {8, 8, box_chunks} lands as box_chunks
 // consecutive 128-byte core matrices of 8 rows.  Rows past `rows` and chunks past `chunks` read
 // as zeros.  The encoder takes the non-monotonic strides (checked on GB300: bit-exact layout).
+// With more rows per box the row groups of a chunk follow one another (128 bytes apart) and the
+// chunks lie box_rows * 16 bytes apart.
 inline int tensor_map_kmajor_groups(CUtensorMap* map, const void* base, int64_t rows, int64_t chunks, int64_t ld,
-                                    int box_chunks, const char* what) {
+                                    int box_chunks, const char* what, int box_rows = 8) {
     PFN_cuTensorMapEncodeTiled_v12000 enc = tensor_map_encoder();
     if (!enc) {
         set_error("cuTensorMapEncodeTiled is not available from the driver");
@@ -64,7 +66,7 @@ inline int tensor_map_kmajor_groups(CUtensorMap* map, const void* base, int64_t 
     }
     const cuuint64_t dims[3] = {8, (cuuint64_t)rows, (cuuint64_t)chunks};
     const cuuint64_t strides[2] = {(cuuint64_t)ld * 2, 16};
-    const cuuint32_t box[3] = {8, 8, (cuuint32_t)box_chunks};
+    const cuuint32_t box[3] = {8, (cuuint32_t)box_rows, (cuuint32_t)box_chunks};
     const cuuint32_t es[3] = {1, 1, 1};
     const CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void*>(base), dims, strides, box, es,
                            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
