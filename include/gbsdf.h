@@ -422,7 +422,7 @@ int gbsdf_mesh_finalize(const double* V, int64_t nv, const int64_t* F, int64_t n
  * application that owns the device budget and forbids allocations after
  * start-up, or a latency-critical loop where cudaMalloc/cudaFree could
  * synchronise the device.  Same inputs, outputs and results as gbsdf_mc_block,
- * but the scratch lives in a fixed 12.5 MiB file-scope device array of this
+ * but the scratch lives in a fixed 247 KiB file-scope device array of this
  * library, so blocks are limited to 33 x 33 x 33 points (larger ones are
  * rejected with GBSDF_ERR_ARG).  The first call on a device looks up the
  * array's device address (make it before any stream capture).  All calls share

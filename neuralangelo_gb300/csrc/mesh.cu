@@ -4,23 +4,21 @@
 //   marching_cubes (:119-133)           -> PyMCubes on the CPU, then V * intv + xyz[0,0,0]
 //   filter_points_outside_bounding_sphere (:136-148)
 // Here one block volume [nx, ny, nz] (float32, x-major, already negated as
-// scripts/extract_mesh.py:85 does) goes through count -> exclusive scan -> emit
+// scripts/extract_mesh.py:85 does) goes through classify -> exclusive scan -> emit
 // on the device:
-//   1. crossing edges (grid edge (i,j,k,axis) whose end values straddle iso)
-//      -> vertex numbers in global edge order ((i*ny + j)*nz + k)*3 + axis;
-//   2. cube configurations -> triangle counts -> triangle offsets in x-major
-//      cube order;
-//   3. vertices (double: t = (iso - v0) / (v1 - v0), index-space position,
-//      * intv + origin) and faces from the case table;
-//   4. the unit-sphere filter: keep |v| < 1, keep faces whose vertices are all
-//      kept, re-index by exclusive scans.
+//   1. crossing edges (grid edge (i,j,k,axis) whose end values straddle iso) whose vertex
+//      passes the unit-sphere filter (|v| < 1); the vertex in double: t = (iso - v0) /
+//      (v1 - v0), index-space position, * intv + origin;
+//   2. triangles of every cube whose vertices are all kept, from the case table;
+//   3. sums per block of points, scanned: vertices are numbered in global edge order
+//      ((i*ny + j)*nz + k)*3 + axis, faces in x-major cube order;
+//   4. vertices and faces.
 // The case table follows the canonical triangulation stated in oracle/mc.c
 // (face walks with positive corners separated on ambiguous faces, loops fanned
 // from their smallest edge id); it is generated on the host at first use.
 #include <mutex>
 
 #include "common.cuh"
-#include "scan.cuh"
 
 namespace gbsdf {
 
@@ -138,150 +136,287 @@ __device__ __forceinline__ int64_t vol_index(const McDims& d, int i, int j, int 
     return ((int64_t)i * d.ny + j) * d.nz + k;
 }
 
-__global__ void k_mc_edges(const float* __restrict__ vol, McDims d, double iso, int64_t* __restrict__ flag) {
-    const int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    const int64_t ne = (int64_t)d.nx * d.ny * d.nz * 3;
-    if (g >= ne) return;
-    const int a = (int)(g % 3);
-    const int64_t p = g / 3;
-    const int k = (int)(p % d.nz), j = (int)((p / d.nz) % d.ny), i = (int)(p / ((int64_t)d.ny * d.nz));
-    const int i1 = i + (a == 0), j1 = j + (a == 1), k1 = k + (a == 2);
-    int64_t f = 0;
-    if (i1 < d.nx && j1 < d.ny && k1 < d.nz) {
-        const bool p0 = (double)vol[vol_index(d, i, j, k)] > iso;
-        const bool p1 = (double)vol[vol_index(d, i1, j1, k1)] > iso;
-        f = p0 != p1;
+constexpr int MC_T = 512;        // lattice points per thread block
+
+// One lattice point per thread throughout: the point owns its three edges (towards +x, +y, +z)
+// and the cube at its +x +y +z side, so that point order is edge order and cube order at once.
+struct McPoint {
+    int i, j, k;
+    bool live;
+};
+__device__ __forceinline__ McPoint mc_point(const McDims& d, uint32_t p, uint32_t np) {
+    McPoint q;
+    q.live = p < np;
+    const uint32_t ij = p / (uint32_t)d.nz;
+    q.k = (int)(p - ij * (uint32_t)d.nz);
+    q.i = (int)(ij / (uint32_t)d.ny);
+    q.j = (int)(ij - (uint32_t)q.i * (uint32_t)d.ny);
+    return q;
+}
+__device__ __forceinline__ bool mc_has_cube(const McDims& d, const McPoint& q) {
+    return q.i + 1 < d.nx && q.j + 1 < d.ny && q.k + 1 < d.nz;
+}
+// iso rounded down to float: a float lies above it exactly when it lies above iso (the chip has
+// little double arithmetic, and this comparison runs for every point)
+__device__ __forceinline__ float mc_iso(double iso) { return __double2float_rd(iso); }
+
+// the vertex on the edge along axis a: t = (iso - v0) / (v1 - v0) in double, index space * intv + origin
+struct McGeometry {
+    double iso, intv, org[3];
+};
+__device__ __forceinline__ void mc_vertex(const McGeometry& g, const McPoint& q, int a, float f0, float f1, double* x) {
+    const double v0 = f0, v1 = f1;
+    const double t = __ddiv_rn(__dsub_rn(g.iso, v0), __dsub_rn(v1, v0));
+    const double idx[3] = {(double)q.i, (double)q.j, (double)q.k};
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+        x[c] = __dadd_rn(__dmul_rn(c == a ? __dadd_rn(idx[c], t) : idx[c], g.intv), g.org[c]);
+}
+
+// unit-sphere filter (mesh.py:136-148): |v| < 1 in double.  Both ends of the edge inside a
+// slightly smaller sphere decide it without the double arithmetic (a vertex of finite values lies
+// between them), which the chip has little of.
+__device__ __forceinline__ bool mc_keeps(const McGeometry& g, const McPoint& q, int a, float f0, float f1) {
+    if (isfinite(f0) && isfinite(f1)) {
+        const float intv = (float)g.intv;
+        float r0 = 0.0f, r1 = 0.0f;
+        const int idx[3] = {q.i, q.j, q.k};
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const float x0 = (float)idx[c] * intv + (float)g.org[c], x1 = (float)(idx[c] + (c == a)) * intv + (float)g.org[c];
+            r0 = fmaf(x0, x0, r0);
+            r1 = fmaf(x1, x1, r1);
+        }
+        // (float coordinates below 1 built from at most 2^28 steps: off by less than 1e-3 unless origin
+        // and steps nearly cancel, which the bound on the origin rules out)
+        if (r0 < 0.99f && r1 < 0.99f && fabs(g.org[0]) < 1e3 && fabs(g.org[1]) < 1e3 && fabs(g.org[2]) < 1e3) return true;
     }
-    flag[g] = f;
+    double x[3];
+    mc_vertex(g, q, a, f0, f1, x);
+    return __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(x[0], x[0]), __dmul_rn(x[1], x[1])), __dmul_rn(x[2], x[2]))) < 1.0;
 }
 
-__global__ void k_mc_cubes(const float* __restrict__ vol, McDims d, double iso, int64_t* __restrict__ tri_count) {
-    const int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    const int64_t nc = (int64_t)(d.nx - 1) * (d.ny - 1) * (d.nz - 1);
-    if (c >= nc) return;
-    const int k = (int)(c % (d.nz - 1)), j = (int)((c / (d.nz - 1)) % (d.ny - 1)),
-              i = (int)(c / ((int64_t)(d.ny - 1) * (d.nz - 1)));
-    int cfg = 0;
+// sum over the block; every thread's `before` is the sum over earlier threads
+__device__ __forceinline__ uint32_t mc_block_scan(uint32_t v, uint32_t* warp_s, uint32_t& before) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t x = v;
 #pragma unroll
-    for (int q = 0; q < 8; ++q)
-        if ((double)vol[vol_index(d, i + (q & 1), j + ((q >> 1) & 1), k + ((q >> 2) & 1))] > iso) cfg |= 1 << q;
-    tri_count[c] = c_count[cfg];
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+    }
+    if (lane == 31) warp_s[warp] = x;
+    __syncthreads();
+    uint32_t total = 0;
+    before = x - v;
+#pragma unroll
+    for (int w = 0; w < MC_T / 32; ++w) {
+        before += w < warp ? warp_s[w] : 0u;
+        total += warp_s[w];
+    }
+    return total;
 }
 
-__global__ void k_mc_vertices(const float* __restrict__ vol, McDims d, double iso, const int64_t* __restrict__ flag,
-                              const int64_t* __restrict__ vidx, double ox, double oy, double oz, double intv,
-                              double* __restrict__ V) {
-    const int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    const int64_t ne = (int64_t)d.nx * d.ny * d.nz * 3;
-    if (g >= ne || !flag[g]) return;
-    const int a = (int)(g % 3);
-    const int64_t p = g / 3;
-    const int k = (int)(p % d.nz), j = (int)((p / d.nz) % d.ny), i = (int)(p / ((int64_t)d.ny * d.nz));
-    const double v0 = vol[vol_index(d, i, j, k)];
-    const double v1 = vol[vol_index(d, i + (a == 0), j + (a == 1), k + (a == 2))];
-    const double t = __ddiv_rn(__dsub_rn(iso, v0), __dsub_rn(v1, v0));
-    double idx[3] = {(double)i, (double)j, (double)k};
-    idx[a] = __dadd_rn(idx[a], t);
-    const double org[3] = {ox, oy, oz};
-    const int64_t v = vidx[g];
+// 1: the kept crossing edges of every point (bits 0-2 of code), whether its cube has triangles
+// (bit 3) and which (cfg); kept vertices per block
+__global__ void __launch_bounds__(MC_T) k_mc_classify(const float* __restrict__ vol, McDims d, McGeometry g, uint32_t np,
+                                                      uint8_t* __restrict__ code, uint8_t* __restrict__ cfg,
+                                                      uint2* __restrict__ sums) {
+    __shared__ uint32_t warp_s[MC_T / 32];
+    const uint32_t p = blockIdx.x * (uint32_t)MC_T + threadIdx.x;
+    const McPoint q = mc_point(d, p, np);
+    const float iso = mc_iso(g.iso);
+    uint32_t bits = 0;
+    if (q.live) {
+        const int64_t step[3] = {(int64_t)d.ny * d.nz, d.nz, 1};
+        const bool has[3] = {q.i + 1 < d.nx, q.j + 1 < d.ny, q.k + 1 < d.nz};
+        const float f0 = vol[p];
+        float f1[3];
 #pragma unroll
-    for (int q = 0; q < 3; ++q) V[3 * v + q] = __dadd_rn(__dmul_rn(idx[q], intv), org[q]);
+        for (int a = 0; a < 3; ++a) f1[a] = has[a] ? vol[p + step[a]] : f0;
+        if (has[0] && has[1] && has[2]) {
+            // corner c: +1 along axis a where bit a is set
+            const int c = (f0 > iso) | (f1[0] > iso) << 1 | (f1[1] > iso) << 2 | (f1[2] > iso) << 4 |
+                          (vol[p + step[0] + step[1]] > iso) << 3 | (vol[p + step[0] + step[2]] > iso) << 5 |
+                          (vol[p + step[1] + step[2]] > iso) << 6 | (vol[p + step[0] + step[1] + step[2]] > iso) << 7;
+            if (c != 0 && c != 255) {
+                bits = 8u;
+                cfg[p] = (uint8_t)c;
+            }
+        }
+#pragma unroll
+        for (int a = 0; a < 3; ++a)
+            if ((f0 > iso) != (f1[a] > iso) && mc_keeps(g, q, a, f0, f1[a])) bits |= 1u << a;
+        code[p] = (uint8_t)bits;
+    }
+    uint32_t before;
+    const uint32_t t = mc_block_scan(__popc(bits & 7u), warp_s, before);
+    if (threadIdx.x == 0) sums[blockIdx.x].x = t;
 }
 
-__global__ void k_mc_faces(const float* __restrict__ vol, McDims d, double iso, const int64_t* __restrict__ tri_off,
-                           const int64_t* __restrict__ vidx, int64_t* __restrict__ F) {
-    const int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    const int64_t nc = (int64_t)(d.nx - 1) * (d.ny - 1) * (d.nz - 1);
-    if (c >= nc) return;
-    const int k = (int)(c % (d.nz - 1)), j = (int)((c / (d.nz - 1)) % (d.ny - 1)),
-              i = (int)(c / ((int64_t)(d.ny - 1) * (d.nz - 1)));
-    int cfg = 0;
+// Steps 2, 4 and 5 first list the block's items (few: the surface passes through), then take one
+// per thread: spread over the points, a warp would run the table walk or the double division for a
+// lane or two.
+
+// 2: kept triangles of every cube (tri[p], a bit each, in table order) and per block
+__global__ void __launch_bounds__(MC_T) k_mc_count_faces(McDims d, uint32_t np, const uint8_t* __restrict__ code,
+                                                         const uint8_t* __restrict__ cfg, uint8_t* __restrict__ tri,
+                                                         uint2* __restrict__ sums) {
+    __shared__ uint32_t warp_s[MC_T / 32];
+    __shared__ uint16_t list[MC_T];
+    __shared__ uint32_t faces;
+    const uint32_t p0 = blockIdx.x * (uint32_t)MC_T, p = p0 + threadIdx.x;
+    const bool active = p < np && (code[p] & 8u);
+    if (p < np && !active) tri[p] = 0;
+    if (threadIdx.x == 0) faces = 0;
+    uint32_t at;
+    const uint32_t n = mc_block_scan(active, warp_s, at);
+    if (active) list[at] = (uint16_t)threadIdx.x;
+    __syncthreads();
+    if (threadIdx.x < n) {
+        const uint32_t pt = p0 + list[threadIdx.x];
+        const McPoint q = mc_point(d, pt, np);
+        const int c = cfg[pt];
+        // the kept vertices of the cube's twelve edges
+        uint32_t edges = 0;
 #pragma unroll
-    for (int q = 0; q < 8; ++q)
-        if ((double)vol[vol_index(d, i + (q & 1), j + ((q >> 1) & 1), k + ((q >> 2) & 1))] > iso) cfg |= 1 << q;
-    const int nt = c_count[cfg];
-    int64_t o = tri_off[c];
-    for (int t = 0; t < nt; ++t, ++o) {
-#pragma unroll
-        for (int q = 0; q < 3; ++q) {
+        for (int e = 0; e < 12; ++e) {
             int a, dx, dy, dz;
-            edge_lo_corner(c_tri[cfg][t][q], a, dx, dy, dz);
-            const int64_t g = vol_index(d, i + dx, j + dy, k + dz) * 3 + a;
-            F[3 * o + q] = vidx[g];
+            edge_lo_corner(e, a, dx, dy, dz);
+            edges |= ((uint32_t)(code[vol_index(d, q.i + dx, q.j + dy, q.k + dz)] >> a) & 1u) << e;
+        }
+        uint32_t kept = 0;
+        const int nt = c_count[c];
+        for (int t = 0; t < nt; ++t) {
+            const uint32_t need = 1u << c_tri[c][t][0] | 1u << c_tri[c][t][1] | 1u << c_tri[c][t][2];
+            if ((edges & need) == need) kept |= 1u << t;
+        }
+        tri[pt] = (uint8_t)kept;
+        if (kept) atomicAdd(&faces, (uint32_t)__popc(kept));
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) sums[blockIdx.x].y = faces;
+}
+
+// 3: exclusive sums over the blocks (one thread block, eight entries per thread and round)
+constexpr int MC_SCAN_T = 1024, MC_SCAN_PER = 8;
+__global__ void __launch_bounds__(MC_SCAN_T) k_mc_scan_blocks(uint2* __restrict__ sums, uint32_t nb,
+                                                              int64_t* __restrict__ counts) {
+    __shared__ uint2 warp_s[MC_SCAN_T / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint2 carry = make_uint2(0, 0);
+    for (uint32_t base = 0; base < nb; base += MC_SCAN_T * MC_SCAN_PER) {
+        const uint32_t at = base + threadIdx.x * MC_SCAN_PER;
+        uint2 v[MC_SCAN_PER], sum = make_uint2(0, 0);
+#pragma unroll
+        for (int i = 0; i < MC_SCAN_PER; ++i) {
+            v[i] = at + i < nb ? sums[at + i] : make_uint2(0, 0);
+            sum.x += v[i].x;
+            sum.y += v[i].y;
+        }
+        uint2 x = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t yx = __shfl_up_sync(0xffffffffu, x.x, o), yy = __shfl_up_sync(0xffffffffu, x.y, o);
+            if (lane >= o) {
+                x.x += yx;
+                x.y += yy;
+            }
+        }
+        if (lane == 31) warp_s[warp] = x;
+        __syncthreads();
+        uint2 before = carry;
+        for (int w = 0; w < MC_SCAN_T / 32; ++w) {
+            const uint2 t = warp_s[w];
+            if (w < warp) {
+                before.x += t.x;
+                before.y += t.y;
+            }
+            carry.x += t.x;
+            carry.y += t.y;
+        }
+        before.x += x.x - sum.x;
+        before.y += x.y - sum.y;
+#pragma unroll
+        for (int i = 0; i < MC_SCAN_PER; ++i) {
+            if (at + i < nb) sums[at + i] = before;
+            before.x += v[i].x;
+            before.y += v[i].y;
+        }
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+        counts[0] = carry.x;
+        counts[1] = carry.y;
+    }
+}
+
+// 4: kept vertices, and the number of each point's first one
+__global__ void __launch_bounds__(MC_T) k_mc_vertices(const float* __restrict__ vol, McDims d, McGeometry g, uint32_t np,
+                                                      const uint8_t* __restrict__ code, const uint2* __restrict__ sums,
+                                                      uint32_t* __restrict__ first, double* __restrict__ V) {
+    __shared__ uint32_t warp_s[MC_T / 32];
+    __shared__ uint16_t list[3 * MC_T];
+    const uint32_t p0 = blockIdx.x * (uint32_t)MC_T, p = p0 + threadIdx.x;
+    const uint32_t bits = p < np ? code[p] & 7u : 0u, v0 = sums[blockIdx.x].x;
+    uint32_t at;
+    const uint32_t n = mc_block_scan(__popc(bits), warp_s, at);
+    if (bits) first[p] = v0 + at;
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+        if ((bits >> a) & 1u) list[at++] = (uint16_t)(threadIdx.x * 3 + a);
+    __syncthreads();
+    for (uint32_t r = threadIdx.x; r < n; r += MC_T) {
+        const uint32_t lp = list[r] / 3u, a = list[r] - 3u * lp, pt = p0 + lp;
+        const McPoint q = mc_point(d, pt, np);
+        const int64_t step = a == 0 ? (int64_t)d.ny * d.nz : a == 1 ? d.nz : 1;
+        double x[3];
+        mc_vertex(g, q, (int)a, vol[pt], vol[pt + step], x);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) V[3 * ((int64_t)v0 + r) + c] = x[c];
+    }
+}
+
+// 5: kept faces
+__global__ void __launch_bounds__(MC_T) k_mc_faces(McDims d, uint32_t np, const uint8_t* __restrict__ code,
+                                                   const uint8_t* __restrict__ cfg, const uint8_t* __restrict__ tri,
+                                                   const uint2* __restrict__ sums, const uint32_t* __restrict__ first,
+                                                   int64_t* __restrict__ F) {
+    __shared__ uint32_t warp_s[MC_T / 32];
+    __shared__ uint16_t list[5 * MC_T];
+    const uint32_t p0 = blockIdx.x * (uint32_t)MC_T, p = p0 + threadIdx.x;
+    const uint32_t kept = p < np ? tri[p] : 0u;
+    const int64_t o0 = sums[blockIdx.x].y;
+    uint32_t at;
+    const uint32_t n = mc_block_scan(__popc(kept), warp_s, at);
+    for (uint32_t left = kept; left; left &= left - 1) list[at++] = (uint16_t)(threadIdx.x * 8 + __ffs(left) - 1);
+    __syncthreads();
+    for (uint32_t r = threadIdx.x; r < n; r += MC_T) {
+        const uint32_t pt = p0 + (list[r] >> 3), t = list[r] & 7u;
+        const McPoint q = mc_point(d, pt, np);
+        const int8_t* tr = c_tri[cfg[pt]][t];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            int a, dx, dy, dz;
+            edge_lo_corner(tr[c], a, dx, dy, dz);
+            const int64_t m = vol_index(d, q.i + dx, q.j + dy, q.k + dz);
+            F[3 * (o0 + r) + c] = (int64_t)first[m] + __popc(code[m] & ((1u << a) - 1u));
         }
     }
 }
 
-// unit-sphere filter (mesh.py:136-148)
-__global__ void k_keep_vertices(const double* __restrict__ V, const int64_t* __restrict__ nv, int64_t* __restrict__ keep,
-                                int64_t cap) {
-    const int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (v >= cap) return;
-    int64_t k = 0;
-    if (v < *nv) {
-        const double x = V[3 * v], y = V[3 * v + 1], z = V[3 * v + 2];
-        k = __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(x, x), __dmul_rn(y, y)), __dmul_rn(z, z))) < 1.0;
-    }
-    keep[v] = k;
-}
-
-__global__ void k_keep_faces(const int64_t* __restrict__ F, const int64_t* __restrict__ nf,
-                             const int64_t* __restrict__ vkeep, int64_t* __restrict__ fkeep, int64_t cap) {
-    const int64_t f = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (f >= cap) return;
-    int64_t k = 0;
-    if (f < *nf) k = vkeep[F[3 * f]] && vkeep[F[3 * f + 1]] && vkeep[F[3 * f + 2]];
-    fkeep[f] = k;
-}
-
-__global__ void k_compact(const double* __restrict__ V, const int64_t* __restrict__ vkeep,
-                          const int64_t* __restrict__ vnew, int64_t vcap, const int64_t* __restrict__ F,
-                          const int64_t* __restrict__ fkeep, const int64_t* __restrict__ fnew, int64_t fcap,
-                          double* __restrict__ Vout, int64_t* __restrict__ Fout) {
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i < vcap && vkeep[i]) {
-        const int64_t o = vnew[i];
-        Vout[3 * o] = V[3 * i];
-        Vout[3 * o + 1] = V[3 * i + 1];
-        Vout[3 * o + 2] = V[3 * i + 2];
-    }
-    if (i < fcap && fkeep[i]) {
-        const int64_t o = fnew[i];
-#pragma unroll
-        for (int q = 0; q < 3; ++q) Fout[3 * o + q] = vnew[F[3 * i + q]];
-    }
-}
-
-__global__ void k_counts(const int64_t* __restrict__ vnew, const int64_t* __restrict__ vkeep, int64_t vcap,
-                         const int64_t* __restrict__ fnew, const int64_t* __restrict__ fkeep, int64_t fcap,
-                         int64_t* __restrict__ counts) {
-    counts[0] = vcap > 0 ? vnew[vcap - 1] + vkeep[vcap - 1] : 0;
-    counts[1] = fcap > 0 ? fnew[fcap - 1] + fkeep[fcap - 1] : 0;
-}
-
 struct McWorkspace {
-    int64_t* eflag;   // [ne]
-    int64_t* vidx;    // [ne]
-    int64_t* tcount;  // [nc]
-    int64_t* toff;    // [nc]
-    int64_t* raw_n;   // [2] vertices, faces before the filter
-    double* Vraw;     // [vcap, 3]
-    int64_t* Fraw;    // [fcap, 3]
-    int64_t* vkeep;   // [vcap]
-    int64_t* vnew;    // [vcap]
-    int64_t* fkeep;   // [fcap]
-    int64_t* fnew;    // [fcap]
-    int64_t* scan;    // scan scratch
+    uint8_t* code;     // [points] kept edges, cube with triangles
+    uint8_t* cfg;      // [points] corner signs of a cube with triangles
+    uint8_t* tri;      // [points] kept triangles of the cube
+    uint32_t* first;   // [points] number of the point's first kept vertex
+    uint2* sums;       // [blocks] kept vertices and faces, then those of earlier blocks
 };
 
 static size_t align256(size_t b) { return (b + 255) / 256 * 256; }
 
-static size_t mc_layout(int nx, int ny, int nz, int64_t vcap, int64_t fcap, uint8_t* base, McWorkspace* w) {
-    const int64_t ne = (int64_t)nx * ny * nz * 3;
-    const int64_t nc = (int64_t)(nx - 1) * (ny - 1) * (nz - 1);
-    int64_t mx = ne > nc ? ne : nc;
-    if (vcap > mx) mx = vcap;
-    if (fcap > mx) mx = fcap;
+static size_t mc_layout(int nx, int ny, int nz, uint8_t* base, McWorkspace* w) {
+    const size_t np = (size_t)nx * ny * nz, nb = (np + MC_T - 1) / MC_T;
     size_t off = 0;
     auto take = [&](size_t bytes) {
         uint8_t* p = base ? base + off : nullptr;
@@ -289,18 +424,11 @@ static size_t mc_layout(int nx, int ny, int nz, int64_t vcap, int64_t fcap, uint
         return p;
     };
     McWorkspace t;
-    t.eflag = (int64_t*)take(8 * (size_t)ne);
-    t.vidx = (int64_t*)take(8 * (size_t)ne);
-    t.tcount = (int64_t*)take(8 * (size_t)nc);
-    t.toff = (int64_t*)take(8 * (size_t)nc);
-    t.raw_n = (int64_t*)take(16);
-    t.Vraw = (double*)take(24 * (size_t)vcap);
-    t.Fraw = (int64_t*)take(24 * (size_t)fcap);
-    t.vkeep = (int64_t*)take(8 * (size_t)vcap);
-    t.vnew = (int64_t*)take(8 * (size_t)vcap);
-    t.fkeep = (int64_t*)take(8 * (size_t)fcap);
-    t.fnew = (int64_t*)take(8 * (size_t)fcap);
-    t.scan = (int64_t*)take(8 * scan_ws_elems(mx));
+    t.code = take(np);
+    t.cfg = take(np);
+    t.tri = take(np);
+    t.first = (uint32_t*)take(4 * np);
+    t.sums = (uint2*)take(8 * nb);
     if (w) *w = t;
     return off;
 }
@@ -309,30 +437,20 @@ static size_t mc_layout(int nx, int ny, int nz, int64_t vcap, int64_t fcap, uint
 static int64_t mc_vcap(int nx, int ny, int nz) { return (int64_t)nx * ny * nz * 3; }
 static int64_t mc_fcap(int nx, int ny, int nz) { return 5 * (int64_t)(nx - 1) * (ny - 1) * (nz - 1); }
 
+// One pass over the volume classifies every point, two passes over one byte per point emit.
+// Counting per edge and per cube into int64 arrays, scanning those and the worst-case vertex and
+// face lists (30 launches) took 621 us for a 129^3 block, the scans alone 321; this MC_TIMES.
 static int mc_run(const float* vol, int nx, int ny, int nz, double iso, const double* origin, double intv,
                   const McWorkspace& w, double* V, int64_t* F, int64_t* counts, cudaStream_t s) {
     const McDims d{nx, ny, nz};
-    const int64_t ne = (int64_t)nx * ny * nz * 3;
-    const int64_t nc = (int64_t)(nx - 1) * (ny - 1) * (nz - 1);
-    const int64_t vcap = mc_vcap(nx, ny, nz), fcap = mc_fcap(nx, ny, nz);
-    const int T = 256;
-    k_mc_edges<<<(unsigned)((ne + T - 1) / T), T, 0, s>>>(vol, d, iso, w.eflag);
-    exclusive_scan(w.eflag, w.vidx, ne, w.scan, nullptr, s);
-    k_mc_cubes<<<(unsigned)((nc + T - 1) / T), T, 0, s>>>(vol, d, iso, w.tcount);
-    exclusive_scan(w.tcount, w.toff, nc, w.scan, nullptr, s);
-    // counts before the filter: last offset + last count
-    k_counts<<<1, 1, 0, s>>>(w.vidx, w.eflag, ne, w.toff, w.tcount, nc, w.raw_n);
-    k_mc_vertices<<<(unsigned)((ne + T - 1) / T), T, 0, s>>>(vol, d, iso, w.eflag, w.vidx, origin[0], origin[1],
-                                                              origin[2], intv, w.Vraw);
-    k_mc_faces<<<(unsigned)((nc + T - 1) / T), T, 0, s>>>(vol, d, iso, w.toff, w.vidx, w.Fraw);
-    k_keep_vertices<<<(unsigned)((vcap + T - 1) / T), T, 0, s>>>(w.Vraw, w.raw_n, w.vkeep, vcap);
-    exclusive_scan(w.vkeep, w.vnew, vcap, w.scan, nullptr, s);
-    k_keep_faces<<<(unsigned)((fcap + T - 1) / T), T, 0, s>>>(w.Fraw, w.raw_n + 1, w.vkeep, w.fkeep, fcap);
-    exclusive_scan(w.fkeep, w.fnew, fcap, w.scan, nullptr, s);
-    const int64_t mx = vcap > fcap ? vcap : fcap;
-    k_compact<<<(unsigned)((mx + T - 1) / T), T, 0, s>>>(w.Vraw, w.vkeep, w.vnew, vcap, w.Fraw, w.fkeep, w.fnew, fcap,
-                                                         V, F);
-    k_counts<<<1, 1, 0, s>>>(w.vnew, w.vkeep, vcap, w.fnew, w.fkeep, fcap, counts);
+    const McGeometry g{iso, intv, {origin[0], origin[1], origin[2]}};
+    // at most 2^28 points (checked by the entry points): vertices and faces below 2^32
+    const uint32_t np = (uint32_t)((int64_t)nx * ny * nz), nb = (np + MC_T - 1) / MC_T;
+    k_mc_classify<<<nb, MC_T, 0, s>>>(vol, d, g, np, w.code, w.cfg, w.sums);
+    k_mc_count_faces<<<nb, MC_T, 0, s>>>(d, np, w.code, w.cfg, w.tri, w.sums);
+    k_mc_scan_blocks<<<1, MC_SCAN_T, 0, s>>>(w.sums, nb, counts);
+    k_mc_vertices<<<nb, MC_T, 0, s>>>(vol, d, g, np, w.code, w.sums, w.first, V);
+    k_mc_faces<<<nb, MC_T, 0, s>>>(d, np, w.code, w.cfg, w.tri, w.sums, w.first, F);
     return launch_status("marching_cubes");
 }
 
@@ -354,7 +472,7 @@ extern "C" int gbsdf_mc_table(int32_t* tri, int32_t* count) {
 
 extern "C" size_t gbsdf_mc_workspace_size(int nx, int ny, int nz) {
     if (nx < 2 || ny < 2 || nz < 2) return 0;
-    return mc_layout(nx, ny, nz, mc_vcap(nx, ny, nz), mc_fcap(nx, ny, nz), nullptr, nullptr);
+    return mc_layout(nx, ny, nz, nullptr, nullptr);
 }
 
 extern "C" int gbsdf_mc_block(const float* vol, int nx, int ny, int nz, double iso, const double* origin, double intv,
@@ -371,7 +489,7 @@ extern "C" int gbsdf_mc_block(const float* vol, int nx, int ny, int nz, double i
     GBSDF_CHECK_ARG(aligned(workspace, 256), "workspace must be 256-byte aligned");
     if (int st = upload_table_once()) return st;
     McWorkspace w;
-    mc_layout(nx, ny, nz, mc_vcap(nx, ny, nz), mc_fcap(nx, ny, nz), (uint8_t*)workspace, &w);
+    mc_layout(nx, ny, nz, (uint8_t*)workspace, &w);
     return mc_run(vol, nx, ny, nz, iso, origin, intv, w, V, F, counts, as_stream(stream));
 }
 
@@ -385,7 +503,7 @@ extern "C" int gbsdf_mc_block(const float* vol, int nx, int ny, int nz, double i
 // keeps its scratch in a file-scope __device__ array of fixed size, enough for
 // blocks of up to 33 x 33 x 33 lattice points (32^3 cubes).  The array exists on
 // every device that loads this library, for the life of the process
-// (12.5 MiB).  Host code may not take the array's name as a device address, so
+// (247 KiB).  Host code may not take the array's name as a device address, so
 // the device address is looked up with cudaGetSymbolAddress once per device, on
 // the first call made with that device current; make that first call before any
 // stream capture.  Every call reuses the same array: two calls whose kernels
@@ -394,7 +512,7 @@ extern "C" int gbsdf_mc_block(const float* vol, int nx, int ny, int nz, double i
 // call, so nothing carries over from the previous call.
 
 constexpr int kNoAllocMaxPoints = 33;
-constexpr size_t kNoAllocScratchBytes = 13119488;   // gbsdf_mc_workspace_size(33, 33, 33)
+constexpr size_t kNoAllocScratchBytes = 252928;   // gbsdf_mc_workspace_size(33, 33, 33)
 
 static __device__ __align__(256) uint8_t g_mc_scratch[kNoAllocScratchBytes];
 
@@ -440,6 +558,6 @@ extern "C" int gbsdf_mc_block_noalloc(const float* vol, int nx, int ny, int nz, 
     void* scratch = nullptr;
     if (int st = noalloc_scratch(&scratch)) return st;
     McWorkspace w;
-    mc_layout(nx, ny, nz, mc_vcap(nx, ny, nz), mc_fcap(nx, ny, nz), (uint8_t*)scratch, &w);
+    mc_layout(nx, ny, nz, (uint8_t*)scratch, &w);
     return mc_run(vol, nx, ny, nz, iso, origin, intv, w, V, F, counts, as_stream(stream));
 }

@@ -264,3 +264,25 @@ def test_export_mesh_writes_the_oracle_mesh(tmp_path):
     assert np.array_equal(out.vertices, Vr) and np.array_equal(out.faces, Fr)
     V, F, C = gm.read_ply(tmp_path / "mesh.ply")
     assert C is None and np.array_equal(F, Fr) and np.array_equal(V, Vr.astype(np.float32))
+
+
+@pytest.mark.parametrize("dims,intv,bad", [((5, 33, 70), 0.05, False), ((9, 9, 9), 0.4, False), ((17, 8, 64), 0.03, True),
+                                           ((2, 3, 513), 0.002, False), ((163, 162, 161), 0.0115, False)])
+def test_marching_cubes_of_ragged_blocks_matches_oracle(dims, intv, bad):
+    """Blocks that do not fill the thread blocks, one scan round and more than one, vertices on
+    both sides of the unit sphere, infinite values on crossing edges."""
+    rng = np.random.default_rng(sum(dims))
+    origin = (-0.5 * intv * (np.array(dims) - 1) + 0.1).astype(np.float32)     # the oracle's type
+    g = [origin[a] + intv * np.arange(dims[a]) for a in range(3)]
+    X = np.stack(np.meshgrid(*g, indexing='ij'), -1)
+    vol = (np.sin(7 * X).prod(-1) * 0.3 + 0.2 * rng.normal(size=dims)).astype(np.float32)
+    if np.prod(dims) > 10 ** 6:
+        vol = (0.85 - np.linalg.norm(X, axis=-1) + 0.1 * np.sin(20 * X).prod(-1)).astype(np.float32)
+    if bad:
+        vol[3, 4, 10], vol[9, 2, 33] = np.inf, -np.inf
+    with np.errstate(all='ignore'):
+        Vr, Fr = om.marching_cubes_block(vol, origin, intv)
+    V, F = gm.MarchingCubes(max(dims), DEV)(torch.from_numpy(vol).to(DEV), [float(o) for o in origin], intv)
+    V, F = V.cpu().numpy(), F.cpu().numpy()
+    assert len(Fr) > 0 and np.array_equal(F, Fr)
+    assert V.shape == Vr.shape and np.allclose(V, Vr, rtol=0, atol=1e-12)
