@@ -506,6 +506,21 @@ int gbsdf_weightnorm_bwd(int32_t n, const gbsdf_weightnorm_layer* layers, const 
                          void* stream);
 size_t gbsdf_weightnorm_layer_size(void);   /* sizeof(gbsdf_weightnorm_layer), for binding checks */
 
+/* The same with dW read through a column map, straight from the layout in which the step's kernels
+ * leave it: column dst[s] + i of the layer (0 <= i < n[s]) takes dW column src[s] + i, plus column
+ * src2[s] + i unless src2[s] < 0; columns of no segment have gradient 0.  nseg = 0: column j is
+ * dW column j.  found_inf (optional): set to 1 when a gradient written is not finite (the check
+ * of GradScaler.unscale_ on these parameters). */
+#define GBSDF_WN_MAX_SEGMENTS 4
+typedef struct gbsdf_weightnorm_map {
+    int32_t nseg, pad;
+    int32_t dst[GBSDF_WN_MAX_SEGMENTS], n[GBSDF_WN_MAX_SEGMENTS];
+    int32_t src[GBSDF_WN_MAX_SEGMENTS], src2[GBSDF_WN_MAX_SEGMENTS];
+} gbsdf_weightnorm_map;
+int gbsdf_weightnorm_bwd_mapped(int32_t n, const gbsdf_weightnorm_layer* layers, const gbsdf_weightnorm_map* maps,
+                                const float* scale_dev, float scale, float* found_inf, void* stream);
+size_t gbsdf_weightnorm_map_size(void);
+
 /* Working copies of weight-normalised (or plain) weights for the fused step: per entry, rows of
  * W = g v / ||v|| (the norm over all `cols` of each source row; g == NULL: W = v), columns
  * [col0, col0 + ncols), written to any of: dst16 (fp16, row stride ld16, the segment's first

@@ -23,11 +23,27 @@ namespace {
 
 struct WnParams {
     gbsdf_weightnorm_layer L[GBSDF_WN_MAX_LAYERS];
+    gbsdf_weightnorm_map M[GBSDF_WN_MAX_LAYERS];
     int64_t row0[GBSDF_WN_MAX_LAYERS + 1];   // first global row of each entry; row0[n] = total
     int n;
     const float* scale_dev;                   // device scalar (dynamic loss scaling) or NULL
     float scale;
+    float* found_inf;
 };
+
+constexpr int WN_REG = 12;
+
+// column j of a layer's effective-weight gradient
+__device__ __forceinline__ float wn_dw(const float* dW, const gbsdf_weightnorm_map& m, int64_t j) {
+    if (m.nseg == 0) return dW[j];
+    for (int s = 0; s < m.nseg; ++s) {
+        const int64_t i = j - m.dst[s];
+        if (i < 0 || i >= m.n[s]) continue;
+        const float x = dW[m.src[s] + i];
+        return m.src2[s] >= 0 ? x + dW[m.src2[s] + i] : x;
+    }
+    return 0.0f;
+}
 
 __device__ __forceinline__ float wn_warp_sum(float v) {
 #pragma unroll
@@ -42,39 +58,65 @@ __global__ void __launch_bounds__(256) k_weightnorm_bwd(const __grid_constant__ 
     int l = 0;
     while (grow >= p.row0[l + 1]) ++l;
     const gbsdf_weightnorm_layer& L = p.L[l];
+    const gbsdf_weightnorm_map& M = p.M[l];
     const int64_t r = grow - p.row0[l];
     const int64_t cols = L.cols;
     const float s = p.scale_dev ? *p.scale_dev : p.scale;
     const float* dW = L.dW + r * L.ld_dw;
     float* dv = L.dv + r * cols;
-    if (L.v == nullptr) {
-        for (int64_t j = lane; j < cols; j += 32) {
-            const float x = s * dW[j];
-            dv[j] = L.acc_v ? dv[j] + x : x;
+    bool bad = false;
+    auto put = [&](float* dst, bool acc, float x) {
+        x = acc ? *dst + x : x;
+        bad |= !isfinite(x);
+        *dst = x;
+    };
+    // rows of up to 32 WN_REG columns stay in registers between the sums and the write, all their
+    // loads in flight at once
+    float w[WN_REG], vv[WN_REG];
+    const bool regs = cols <= 32 * WN_REG;
+    if (regs) {
+#pragma unroll
+        for (int i = 0; i < WN_REG; ++i) {
+            const int64_t j = lane + 32 * i;
+            w[i] = j < cols ? wn_dw(dW, M, j) : 0.0f;
+            vv[i] = j < cols && L.v ? L.v[r * cols + j] : 0.0f;
         }
-    } else {
-        const float* v = L.v + r * cols;
+    }
+    float a = 0.0f, b = 0.0f;                            // dv = a (s dW - v b)
+    if (L.v) {
         float n2 = 0.0f, dot = 0.0f;
-        for (int64_t j = lane; j < cols; j += 32) {
-            const float vv = v[j];
-            n2 = fmaf(vv, vv, n2);
-            dot = fmaf(dW[j], vv, dot);
+        if (regs) {
+#pragma unroll
+            for (int i = 0; i < WN_REG; ++i) {
+                n2 = fmaf(vv[i], vv[i], n2);
+                dot = fmaf(w[i], vv[i], dot);
+            }
+        } else {
+            for (int64_t j = lane; j < cols; j += 32) {
+                const float x = L.v[r * cols + j];
+                n2 = fmaf(x, x, n2);
+                dot = fmaf(wn_dw(dW, M, j), x, dot);
+            }
         }
         n2 = wn_warp_sum(n2);
         dot = wn_warp_sum(dot);
         const float n = sqrtf(n2);
         const float dg = s * dot / n;
-        const float a = L.g[r] / n, b = dg / n;
-        for (int64_t j = lane; j < cols; j += 32) {
-            const float x = a * (s * dW[j] - v[j] * b);
-            dv[j] = L.acc_v ? dv[j] + x : x;
-        }
-        if (lane == 0) L.dg[r] = L.acc_g ? L.dg[r] + dg : dg;
+        a = L.g[r] / n;
+        b = dg / n;
+        if (lane == 0) put(L.dg + r, L.acc_g, dg);
     }
-    if (lane == 0 && L.db && L.dbias) {
-        const float x = s * L.db[r * L.ld_db];
-        L.dbias[r] = L.acc_b ? L.dbias[r] + x : x;
+    auto grad = [&](float dw, float x) { return L.v ? a * (s * dw - x * b) : s * dw; };
+    if (regs) {
+#pragma unroll
+        for (int i = 0; i < WN_REG; ++i)
+            if (lane + 32 * i < cols) put(dv + lane + 32 * i, L.acc_v, grad(w[i], vv[i]));
+    } else {
+        for (int64_t j = lane; j < cols; j += 32)
+            put(dv + j, L.acc_v, grad(wn_dw(dW, M, j), L.v ? L.v[r * cols + j] : 0.0f));
     }
+    if (lane == 0 && L.db && L.dbias) put(L.dbias + r, L.acc_b, s * L.db[r * L.ld_db]);
+    if (bad && p.found_inf) *p.found_inf = 1.0f;           // any writer stores the same value
 }
 
 // ---------------------------------------------------------------------------
@@ -152,8 +194,9 @@ extern "C" int gbsdf_weightnorm_fwd(int32_t n, const gbsdf_weightnorm_pack* entr
 
 extern "C" size_t gbsdf_weightnorm_pack_size(void) { return sizeof(gbsdf_weightnorm_pack); }
 
-extern "C" int gbsdf_weightnorm_bwd(int32_t n, const gbsdf_weightnorm_layer* layers, const float* scale_dev,
-                                    float scale, void* stream) {
+extern "C" int gbsdf_weightnorm_bwd_mapped(int32_t n, const gbsdf_weightnorm_layer* layers,
+                                           const gbsdf_weightnorm_map* maps, const float* scale_dev, float scale,
+                                           float* found_inf, void* stream) {
     clear_error();
     GBSDF_CHECK_ARG(n >= 0 && n <= GBSDF_WN_MAX_LAYERS, "n %d (0 to %d entries)", n, GBSDF_WN_MAX_LAYERS);
     GBSDF_CHECK_ARG(n == 0 || layers != nullptr, "NULL layers");
@@ -161,14 +204,25 @@ extern "C" int gbsdf_weightnorm_bwd(int32_t n, const gbsdf_weightnorm_layer* lay
     p.n = n;
     p.scale_dev = scale_dev;
     p.scale = scale;
+    p.found_inf = found_inf;
     int64_t rows = 0;
     for (int i = 0; i < n; ++i) {
         const gbsdf_weightnorm_layer& L = layers[i];
         GBSDF_CHECK_ARG(L.rows >= 0 && L.cols > 0, "entry %d: rows %lld, cols %lld", i, (long long)L.rows,
                         (long long)L.cols);
         GBSDF_CHECK_ARG(L.dW && L.dv, "entry %d: NULL dW or dv", i);
-        GBSDF_CHECK_ARG(L.ld_dw >= L.cols || L.rows <= 1, "entry %d: ld_dw %lld < cols %lld", i, (long long)L.ld_dw,
-                        (long long)L.cols);
+        if (maps) p.M[i] = maps[i];
+        const gbsdf_weightnorm_map& M = p.M[i];
+        GBSDF_CHECK_ARG(M.nseg >= 0 && M.nseg <= GBSDF_WN_MAX_SEGMENTS, "entry %d: %d column segments", i, M.nseg);
+        int64_t need = M.nseg == 0 ? L.cols : 0;           // dW columns read
+        for (int s = 0; s < M.nseg; ++s) {
+            GBSDF_CHECK_ARG(M.dst[s] >= 0 && M.n[s] >= 0 && M.src[s] >= 0 && (int64_t)M.dst[s] + M.n[s] <= L.cols,
+                            "entry %d: column segment %d", i, s);
+            const int64_t last = (int64_t)(M.src2[s] > M.src[s] ? M.src2[s] : M.src[s]) + M.n[s];
+            if (last > need) need = last;
+        }
+        GBSDF_CHECK_ARG(L.ld_dw >= need || L.rows <= 1, "entry %d: ld_dw %lld < %s%lld", i, (long long)L.ld_dw,
+                        M.nseg == 0 ? "cols " : "", (long long)need);
         GBSDF_CHECK_ARG(!L.v || (L.g && L.dg), "entry %d: weight norm needs g and dg", i);
         GBSDF_CHECK_ARG(!L.db || !L.dbias || L.ld_db >= 1 || L.rows <= 1, "entry %d: ld_db %lld", i,
                         (long long)L.ld_db);
@@ -182,5 +236,12 @@ extern "C" int gbsdf_weightnorm_bwd(int32_t n, const gbsdf_weightnorm_layer* lay
     k_weightnorm_bwd<<<(unsigned)blocks, 256, 0, as_stream(stream)>>>(p);
     return launch_status("weightnorm_bwd");
 }
+
+extern "C" int gbsdf_weightnorm_bwd(int32_t n, const gbsdf_weightnorm_layer* layers, const float* scale_dev,
+                                    float scale, void* stream) {
+    return gbsdf_weightnorm_bwd_mapped(n, layers, nullptr, scale_dev, scale, nullptr, stream);
+}
+
+extern "C" size_t gbsdf_weightnorm_map_size(void) { return sizeof(gbsdf_weightnorm_map); }
 
 extern "C" size_t gbsdf_weightnorm_layer_size(void) { return sizeof(gbsdf_weightnorm_layer); }

@@ -140,7 +140,15 @@ class WeightNormLayer(ctypes.Structure):
 
 
 WN_MAX_LAYERS = 16
+WN_MAX_SEGMENTS = 4
 _lib.register("gbsdf_weightnorm_bwd", [c_i32, c_vp, c_vp, c_f32, c_vp])
+_lib.register("gbsdf_weightnorm_bwd_mapped", [c_i32, c_vp, c_vp, c_vp, c_f32, c_vp, c_vp])
+
+
+class WeightNormMap(ctypes.Structure):
+    """gbsdf_weightnorm_map (include/gbsdf.h)."""
+    _fields_ = [("nseg", c_i32), ("pad", c_i32), ("dst", c_i32 * WN_MAX_SEGMENTS), ("n", c_i32 * WN_MAX_SEGMENTS),
+                ("src", c_i32 * WN_MAX_SEGMENTS), ("src2", c_i32 * WN_MAX_SEGMENTS)]
 
 
 class _GradSink:
@@ -164,8 +172,19 @@ class _GradSink:
         return self.seen[key]
 
 
-def _wn_entry(sink, dW, db=None, weight=None, bias=None, v=None, g=None, rows=None):
-    """One gbsdf_weightnorm_layer: the weight-norm parameters v, g (weight-norm entry) or the
+def _mapped(gx, cols, segs):
+    """The [rows, cols] gradient whose columns lie in gx as ``segs`` says: (dst, n, src, src2 or
+    -1) per segment, zero elsewhere (what gbsdf_weightnorm_bwd_mapped reads in place)."""
+    dW = torch.zeros(gx.shape[0], cols, device=gx.device, dtype=gx.dtype)
+    for dst, n, src, src2 in segs:
+        dW[:, dst:dst + n] = gx[:, src:src + n]
+        if src2 >= 0:
+            dW[:, dst:dst + n] += gx[:, src2:src2 + n]
+    return dW
+
+
+def _wn_entry(sink, dW, db=None, weight=None, bias=None, v=None, g=None, rows=None, segs=()):
+    """One gbsdf_weightnorm_layer with its column map ``segs`` (see ``_mapped``; none: dW's own columns): the weight-norm parameters v, g (weight-norm entry) or the
     plain weight (plain entry), the bias, and the row range ``rows`` (a slice of the
     destination's rows, for gradients assembled from row blocks)."""
     if dW.dim() == 1:
@@ -173,6 +192,12 @@ def _wn_entry(sink, dW, db=None, weight=None, bias=None, v=None, g=None, rows=No
     assert dW.stride(1) == 1 and dW.dtype == torch.float32
     e = WeightNormLayer()
     e.rows, e.cols = dW.shape
+    m = WeightNormMap()
+    if segs:
+        e.cols = (v if v is not None else weight).shape[1]
+        m.nseg = len(segs)
+        for i, seg in enumerate(segs):
+            m.dst[i], m.n[i], m.src[i], m.src2[i] = seg
     e.dW, e.ld_dw = dW.data_ptr(), dW.stride(0)
     sl = rows if rows is not None else slice(0, dW.shape[0])
     if v is not None:
@@ -189,6 +214,7 @@ def _wn_entry(sink, dW, db=None, weight=None, bias=None, v=None, g=None, rows=No
         dbias, e.acc_b = sink(bias)
         e.db, e.ld_db = db.data_ptr(), db.stride(0)
         e.dbias = dbias.reshape(-1)[sl].data_ptr()
+    e.colmap = m
     return e
 
 
@@ -250,15 +276,17 @@ def _weightnorm_fwd(entries, device):
         _lib.call("gbsdf_weightnorm_fwd", len(chunk), ctypes.cast(arr, c_vp), _lib.stream_ptr(device))
 
 
-def _weightnorm_bwd(entries, scale, device):
-    """All entries in launches of up to WN_MAX_LAYERS; scale a device scalar or a float."""
+def _weightnorm_bwd(entries, scale, device, found_inf=None):
+    """All entries in launches of up to WN_MAX_LAYERS; scale a device scalar or a float; found_inf
+    a device float set when a gradient written is not finite."""
     sdev = scale.data_ptr() if torch.is_tensor(scale) else None
     sval = 0.0 if torch.is_tensor(scale) else float(scale)
     for i in range(0, len(entries), WN_MAX_LAYERS):
         chunk = entries[i:i + WN_MAX_LAYERS]
         arr = (WeightNormLayer * len(chunk))(*chunk)
-        _lib.call("gbsdf_weightnorm_bwd", len(chunk), ctypes.cast(arr, c_vp), c_vp(sdev), sval,
-                  _lib.stream_ptr(device))
+        maps = (WeightNormMap * len(chunk))(*[e.colmap for e in chunk])
+        _lib.call("gbsdf_weightnorm_bwd_mapped", len(chunk), ctypes.cast(arr, c_vp), ctypes.cast(maps, c_vp),
+                  c_vp(sdev), sval, c_vp(_p(found_inf)), _lib.stream_ptr(device))
 
 
 def active_table_params(sdf):
@@ -529,24 +557,48 @@ class FusedField:
         e = lambda *s, dt=f32: torch.empty(*s, device=device, dtype=dt)  # noqa: E731
         Hc = self.Hc
         ws = dict(key=key)
+        # everything a step adds into, in one buffer cleared by one launch: the device flags and
+        # loss sums first (all that an evaluation needs), then the gradients in the layouts in
+        # which the kernels leave them
+        Kx, dw0 = 2 * self.K0 + 16, self._in_kernel_w0_grad()
+        sums = dict(loss_sums=((4,), torch.float64), err=((1,), torch.int32), d_s_var=((1,), f32))
+        sums.update(d_wl=((3, Hc), f32), d_bl=((3,), f32), d_whead=((256,), f32), d_bhead=((1,), f32),
+                    d_w0=((256, self.K0 + 16 if dw0 else Kx), f32), gw0=((Hc, self.Kc0), f32), gw1=((256, 264), f32))
+        sums.update({f'gw_c{i}': ((Hc, Hc + 8), f32) for i in range(1, self.n_rgb_hidden)})
+        if self.app_dim:
+            sums['g_app'] = (tuple(self.model.appear_embed.weight.shape), f32)
+        if self.bg:
+            Hbr = self.Hbr
+            sums.update(bg_d_bl=((3,), f32), bg_gr1=((3, Hbr), f32), bg_gr0=((Hbr, self.Kr0), f32),
+                        bg_g7=((272, 264), f32), bg_g0=((256, BG_X_COLS), f32), bg_g4=((256, BG_S_COLS), f32))
+            sums.update({f'bg_g{i}': ((256, 264), f32) for i in (1, 2, 3, 5, 6)})
+            if self.app_dim:
+                sums['bg_g_app'] = (tuple(self.model.appear_embed_outside.weight.shape), f32)
+        at = {}
+        size = 0
+        for name, (shape, dt) in sums.items():       # 16-byte aligned pieces
+            at[name] = size
+            size += (int(np.prod(shape)) * dt.itemsize + 15) // 16 * 16
+        arena = torch.zeros(size, device=device, dtype=torch.uint8)
+        ws.update(sums=arena, sums_eval=arena[:at['d_wl']])
+        for name, (shape, dt) in sums.items():
+            n = int(np.prod(shape)) * dt.itemsize
+            ws[name] = arena[at[name]:at[name] + n].view(dt).view(shape)
+        gw0x = ws.pop('d_w0')
+        ws.update(d_w0=gw0x if dw0 else None, gw0x=gw0x)
         ws.update(sdf=e(Ns), grad=e(Ns, 3), hess=e(Ns, 3), h0c=self._with_ones(e(Ns, 264, dt=f16), 256),
                   xc=e(Ns, self.Kc0, dt=f16),
                   ys=[self._with_ones(e(Ns, Hc + 8, dt=f16), Hc) for _ in range(self.n_rgb_hidden)],
                   rgbs=e(Ns, 3), rgb=e(R, 3),
                   weights=e(Ns), d_rgbs=e(Ns, 3), d_sdf=e(Ns), d_grad=e(Ns, 3), d_hess=e(Ns, 3),
-                  loss_sums=torch.zeros(4, device=device, dtype=torch.float64), d_s_var=torch.zeros(1, device=device),
-                  d_wl=torch.zeros(3, Hc, device=device), dzs=[e(Ns, Hc, dt=f16) for _ in range(2)],
+                  dzs=[e(Ns, Hc, dt=f16) for _ in range(2)],
                   dzs_lo=[e(Ns, Hc, dt=f16) for _ in range(2)] if self.split else None,
                   dzfeat=e(Ns, 256, dt=f16), dzfeat_lo=e(Ns, 256, dt=f16) if self.split else None,
                   dxc_tail=e(Ns, 64), d_h0c=e(Ns, 256),
                   # K0 <= 64: the backward kernel accumulates dW0 itself; otherwise d_pre0 -> k_wgrad
                   d_pre0=None if self._in_kernel_w0_grad() else e(rows0, 256, dt=f16),
                   d_pre0_lo=None if self._in_kernel_w0_grad() else e(rows0, 256, dt=f16),
-                  d_w0=e(256, self.K0 + 16) if self._in_kernel_w0_grad() else None,
                   x0ext=e(rows0, 2 * self.K0 + 16, dt=f16), d_enc=e(rows0, self.K0),
-                  d_whead=torch.zeros(256, device=device),
-                  d_bhead=torch.zeros(1, device=device), d_bl=torch.zeros(3, device=device),
-                  err=torch.zeros(1, device=device, dtype=torch.int32),
                   d_table_fix=(torch.empty(wsz.d_table_fix_bytes // 8, device=device, dtype=torch.int64)
                                if self.deterministic else None))
         if self.pairs:
@@ -557,14 +609,13 @@ class FusedField:
             ws.update(h0c_lo=None, xc_lo=None, ys_lo=[None] * (self.n_rgb_hidden - 1))
         if self.bg:
             Nb = R * self.n_bg
-            Hbr = self.Hbr
             ws.update(bg_S=e(Nb, BG_S_COLS, dt=f16),
                       bg_h={i: self._with_ones(e(Nb, 264, dt=f16), 256) for i in (1, 2, 3, 5, 6, 7)},
                       bg_G=e(Nb, self.Kr0, dt=f16), bg_hr=self._with_ones(e(Nb, Hbr + 8, dt=f16), Hbr),
                       bg_sigma=e(Nb), bg_rgbs=e(Nb, 3), bg_weights=e(Nb), bg_d_rgbs=e(Nb, 3),
                       bg_dZ7=torch.zeros(Nb, 272, device=device, dtype=f16), bg_dz_r=e(Nb, Hbr, dt=f16),
                       bg_dz=[e(Nb, 256, dt=f16) for _ in range(2)],
-                      bg_d_tail=e(Nb, 64) if self.app_dim else None, bg_d_bl=torch.zeros(3, device=device))
+                      bg_d_tail=e(Nb, 64) if self.app_dim else None)
             if self.pairs:
                 # low halves of every background activation that feeds another layer's forward
                 # (or the density head); the colour hidden layer feeds the FP32 head only
@@ -639,7 +690,7 @@ class FusedField:
         eps = float(sdfm.normal_eps)
         lay = sdfm.tcnn_encoding.layout
         Hc = self.Hc
-        ws['err'].zero_()
+        (ws['sums_eval'] if _evaluate else ws['sums']).zero_()
 
         fa = FieldArgs()
         fa.Ns, fa.S = Ns, S
@@ -717,8 +768,6 @@ class FusedField:
         ra.rgb, ra.weights = _p(ws['rgb']), _p(ws['weights'])
         ra.d_rgbs, ra.d_sdf, ra.d_grad, ra.d_hess = _p(ws['d_rgbs']), _p(ws['d_sdf']), _p(ws['d_grad']), \
             _p(ws['d_hess'])
-        ws['d_s_var'].zero_()
-        ws['loss_sums'].zero_()
         ra.d_s_var, ra.loss_sums = _p(ws['d_s_var']), _p(ws['loss_sums'])
         ra.err = _p(ws['err'])
         if self.bg:
@@ -736,8 +785,6 @@ class FusedField:
             return ev
         _lib.call("gbsdf_render_fused", ctypes.byref(ra), stream)
         # ---------------- colour MLP backward ----------------
-        ws['d_bl'].zero_()
-        ws['d_wl'].zero_()
         dz = ws['dzs'][0]
         # Y row in, dZ row (and its lo half) out, the per-sample colour and its gradient
         _lib.TIMER.count_bytes("gbsdf_rgb_head_bwd", Ns * (Hc * 2 * (3 if self.split else 2) + 24))
@@ -746,15 +793,14 @@ class FusedField:
                   c_vp(dz.data_ptr()), c_vp(_p(ws['dzs_lo'][0] if self.split else None)), c_vp(ws['d_bl'].data_ptr()),
                   c_vp(ws['d_wl'].data_ptr()), stream)
         grads = {}
-        dev32 = dict(device=dev, dtype=torch.float32)
         n = self.n_rgb_hidden
         # the last colour layer's weight gradient came with its backward
         grads['wl'], grads['bl'] = ws['d_wl'], ws['d_bl']
         cur = 0
         for i in range(n - 1, 0, -1):
             dzi = ws['dzs'][cur]
-            gw = torch.empty(Hc, Hc + 8, **dev32)
-            _wgrad(dzi, ws['ys'][i - 1], Hc, Hc + 8, gw, err=ws['err'])   # column Hc: the bias gradient
+            gw = ws[f'gw_c{i}']
+            _wgrad(dzi, ws['ys'][i - 1], Hc, Hc + 8, gw, accumulate=True, err=ws['err'])   # column Hc: the bias gradient
             grads[f'wc{i}'], grads[f'bc{i}'] = gw[:, :Hc], gw[:, Hc]
             nxt = ws['dzs'][1 - cur]
             _dense(dzi, pk['wcT'][i], Hc, Hc, nxt, epi=EPI_DRELU, G=ws['ys'][i - 1], err=ws['err'],
@@ -763,21 +809,21 @@ class FusedField:
             cur = 1 - cur
         dz0 = ws['dzs'][cur]
         dz0_lo = ws['dzs_lo'][cur] if self.split else None
-        gw0 = torch.empty(Hc, self.Kc0, **dev32)
-        _wgrad(dz0, ws['xc'], Hc, self.Kc0, gw0, err=ws['err'])   # last column: the bias gradient
+        gw0 = ws['gw0']
+        _wgrad(dz0, ws['xc'], Hc, self.Kc0, gw0, accumulate=True, err=ws['err'])   # last column: the bias gradient
         grads['wc0'], grads['bc0'] = gw0, gw0[:, self.Kc0 - 1]
         # input gradient of colour layer 0: feature part through softplus', tail (x, SH, n, app) as is
         _dense(dz0, pk['wc0T_feat'], 256, Hc, ws['dzfeat'], epi=EPI_DSOFTPLUS, beta=fa.beta, G=ws['xc'],
                err=ws['err'], X_lo=dz0_lo, out_lo=ws['dzfeat_lo'] if self.split else None)
         _dense(dz0, pk['wc0T_tail'], 64, Hc, ws['dxc_tail'], epi=EPI_IDENTITY, err=ws['err'], X_lo=dz0_lo)
         # SDF feature layer
-        gw1 = torch.empty(256, 264, **dev32)
-        _wgrad(ws['dzfeat'], ws['h0c'], 256, 264, gw1, err=ws['err'])   # column 256: the bias gradient
+        gw1 = ws['gw1']
+        _wgrad(ws['dzfeat'], ws['h0c'], 256, 264, gw1, accumulate=True, err=ws['err'])   # column 256: the bias gradient
         grads['w1'], grads['b1'] = gw1[:, :256], gw1[:, 256]
         _dense(ws['dzfeat'], pk['w1T'], 256, 256, ws['d_h0c'], epi=EPI_IDENTITY, err=ws['err'],
                X_lo=ws['dzfeat_lo'] if self.split else None)
         if self.app_dim:
-            g_app = torch.zeros_like(pk['app'])
+            g_app = ws['g_app']
             _lib.call("gbsdf_app_grad", R, S, c_vp(_p(offs)), c_vp(app_idx.data_ptr()),
                       c_vp(ws['dxc_tail'].data_ptr()), 64, 22, self.app_dim, c_vp(g_app.data_ptr()), stream)
             grads['app'] = g_app
@@ -795,8 +841,6 @@ class FusedField:
         fa.d_table_scale = 1.0 / self.loss_scale
         fa.d_table_scale_dev = scal[3:4].data_ptr() if scal is not None else None
         fa.found_inf = scal[4:5].data_ptr() if scal is not None else None
-        ws['d_whead'].zero_()
-        ws['d_bhead'].zero_()
         fa.d_sdf, fa.d_grad, fa.d_hess = _p(ws['d_sdf']), _p(ws['d_grad']), _p(ws['d_hess'])
         fa.d_xc, fa.ld_dxc, fa.normal_col = _p(ws['dxc_tail']), 64, 19
         fa.d_h0c = _p(ws['d_h0c'])
@@ -804,18 +848,14 @@ class FusedField:
         fa.d_pre0_lo = _p(ws['d_pre0_lo'])
         fa.d_table_fix = _p(ws['d_table_fix'])
         fa.d_whead, fa.d_bhead = _p(ws['d_whead']), _p(ws['d_bhead'])
-        if ws['d_w0'] is not None:
-            ws['d_w0'].zero_()
         fa.d_w0 = _p(ws['d_w0'])
         _lib.call("gbsdf_field_mlp_bwd", ctypes.byref(fa), stream)    # = gbsdf_field_bwd in two calls
         _lib.call("gbsdf_field_scatter", ctypes.byref(fa), stream)
-        if ws['d_w0'] is not None:
-            grads['w0ext'] = ws['d_w0']                               # [256, K0 + 16], lo folded in
-        else:
-            gw0x = torch.empty(256, 2 * self.K0 + 16, **dev32)
+        grads['w0ext'] = ws['gw0x']                                   # [256, K0 + 16], lo folded in
+        if ws['d_w0'] is None:
             # d_pre as its hi + lo pair against every x0ext column (features hi, tail, features lo)
-            _wgrad(ws['d_pre0'], ws['x0ext'], 256, 2 * self.K0 + 16, gw0x, dZ_lo=ws['d_pre0_lo'], err=ws['err'])
-            grads['w0ext'] = gw0x
+            _wgrad(ws['d_pre0'], ws['x0ext'], 256, 2 * self.K0 + 16, ws['gw0x'], accumulate=True,
+                   dZ_lo=ws['d_pre0_lo'], err=ws['err'])
         grads['table'] = d_table
         if self.bg:
             grads['bg'] = self._background_backward(R, app_idx, stream)
@@ -869,44 +909,37 @@ class FusedField:
         pre-activation (column 256 of the layer-7 gradient buffer); weight gradients
         dZ^T [X | 1] (loss-scaled, FP32)."""
         ws, pk = self.ws, self.pk
-        dev = ws['bg_S'].device
-        dev32 = dict(device=dev, dtype=torch.float32)
         Nb, Hbr, Kr0 = R * self.n_bg, self.Hbr, self.Kr0
         S, G, h, hr = ws['bg_S'], ws['bg_G'], ws['bg_h'], ws['bg_hr']
         dZ7, dz = ws['bg_dZ7'], ws['bg_dz']
         err = ws['err']
-        g = {}
-        ws['bg_d_bl'].zero_()
-        g['r1'] = torch.zeros(3, Hbr, **dev32)
+        g = {i: ws[f'bg_g{i}'] for i in range(8)}
+        g['r0'], g['r1'] = ws['bg_gr0'], ws['bg_gr1']
         dzr_lo, dZ7_lo, dz_lo = ws['bg_dz_r_lo'], ws['bg_dZ7_lo'], ws['bg_dz_lo']
         _lib.call("gbsdf_rgb_head_bwd", Nb, c_vp(hr.data_ptr()), hr.stride(0), Hbr, c_vp(pk['bwr1'].data_ptr()),
                   c_vp(ws['bg_rgbs'].data_ptr()), c_vp(ws['bg_d_rgbs'].data_ptr()), None,
                   c_vp(ws['bg_dz_r'].data_ptr()), c_vp(_p(dzr_lo)), c_vp(ws['bg_d_bl'].data_ptr()),
                   c_vp(g['r1'].data_ptr()), stream)
-        g['r0'] = torch.empty(Hbr, Kr0, **dev32)
-        _wgrad(ws['bg_dz_r'], G, Hbr, Kr0, g['r0'], err=err)                        # bias column 256 + 16 + app
+        _wgrad(ws['bg_dz_r'], G, Hbr, Kr0, g['r0'], accumulate=True, err=err)                        # bias column 256 + 16 + app
         _dense(ws['bg_dz_r'], pk['bwr0T_feat'], 256, Hbr, dZ7, epi=EPI_DRELU, G=G, err=err,   # d feature pre-act
                X_lo=dzr_lo, out_lo=dZ7_lo)
         if self.app_dim:
             _dense(ws['bg_dz_r'], pk['bwr0T_tail'], 64, Hbr, ws['bg_d_tail'], epi=EPI_IDENTITY, err=err,
                    X_lo=dzr_lo)
-            g['app'] = torch.zeros_like(pk['app_bg'])
+            g['app'] = ws['bg_g_app']
             _lib.call("gbsdf_app_grad", R, self.n_bg, None, c_vp(app_idx.data_ptr()),
                       c_vp(ws['bg_d_tail'].data_ptr()), 64, 16, self.app_dim, c_vp(g['app'].data_ptr()), stream)
-        g[7] = torch.empty(272, 264, **dev32)
-        _wgrad(dZ7, h[7], 272, 264, g[7], err=err)
+        _wgrad(dZ7, h[7], 272, 264, g[7], accumulate=True, err=err)
         _dense(dZ7, pk['bw7extT'], 256, 272, dz[0], epi=EPI_DRELU, G=h[7], err=err,       # dZ6
                X_lo=dZ7_lo, out_lo=dz_lo[0])
         cur = 0
         for i, gate in ((6, h[6]), (5, h[5]), (4, S), (3, h[3]), (2, h[2]), (1, h[1])):
             X = S if i == 4 else h[i]
-            g[i] = torch.empty(256, X.shape[1], **dev32)
-            _wgrad(dz[cur], X, 256, X.shape[1], g[i], err=err)
+            _wgrad(dz[cur], X, 256, X.shape[1], g[i], accumulate=True, err=err)
             _dense(dz[cur], pk['bwT'][i], 256, 256, dz[1 - cur], epi=EPI_DRELU, G=gate, err=err,
                    X_lo=dz_lo[cur], out_lo=dz_lo[1 - cur] if i > 1 else None)
             cur = 1 - cur
-        g[0] = torch.empty(256, BG_X_COLS, **dev32)
-        _wgrad(dz[cur], S[:, 256:], 256, BG_X_COLS, g[0], err=err)
+        _wgrad(dz[cur], S[:, 256:], 256, BG_X_COLS, g[0], accumulate=True, err=err)
         return g
 
     def losses(self):
@@ -941,31 +974,25 @@ class FusedField:
         K0 = self.K0
         l0, l1 = sdf.mlp.linears[0], sdf.mlp.linears[1]
         lins = m.neural_rgb.mlp.linears
-        dW0 = torch.zeros_like(l0.weight_v)
         gx = g['w0ext']      # columns: features hi | x,y,z hi, 1, x,y,z lo, 0 [| features lo]
-        dW0[:, 3:3 + A * F] = gx[:, :A * F]
-        if gx.shape[1] > K0 + 16:                      # the k_wgrad path keeps the lo columns apart
-            dW0[:, 3:3 + A * F] += gx[:, K0 + 16:K0 + 16 + A * F]
-        dW0[:, :3] = gx[:, K0:K0 + 3] + gx[:, K0 + 4:K0 + 7]
-        db0 = gx[:, K0 + 3]
-        # colour layer 0: undo the column reordering
+        # (the k_wgrad path keeps the lo columns apart)
+        lo = K0 + 16 if gx.shape[1] > K0 + 16 else -1
+        seg0 = [(0, 3, K0, K0 + 4), (3, A * F, 0, lo)]
+        # colour layer 0: undo the column reordering ([feat 256 | x 3, SH 16, normal 3, app])
         sh = 16
-        Wc0_grad = torch.zeros(lins[0].weight_v.shape, device=dW0.device, dtype=torch.float32)
         gc0 = g['wc0']
-        Wc0_grad[:, 6 + sh:6 + sh + 256] = gc0[:, :256]
-        Wc0_grad[:, 0:3] = gc0[:, 256:259]
-        Wc0_grad[:, 3:3 + sh] = gc0[:, 259:259 + sh]
-        Wc0_grad[:, 3 + sh:6 + sh] = gc0[:, 259 + sh:262 + sh]
+        segc = [(0, 6 + sh, 256, -1), (6 + sh, 256, 0, -1)]
         if self.app_dim:
-            Wc0_grad[:, 6 + sh + 256:] = gc0[:, 262 + sh:262 + sh + self.app_dim]
-        eff = [(l0, dW0, db0), (l1, g['w1'], g['b1']), (lins[0], Wc0_grad, g['bc0'])]
+            segc.append((6 + sh + 256, self.app_dim, 262 + sh, -1))
+        eff = [(l0, gx, gx[:, K0 + 3], seg0), (l1, g['w1'], g['b1'], ()), (lins[0], gc0, g['bc0'], segc)]
         for i in range(1, self.n_rgb_hidden):
-            eff.append((lins[i], g[f'wc{i}'], g[f'bc{i}']))
-        eff.append((lins[-1], g['wl'], g['bl']))
+            eff.append((lins[i], g[f'wc{i}'], g[f'bc{i}'], ()))
+        eff.append((lins[-1], g['wl'], g['bl'], ()))
         names = ['sdf.l0', 'sdf.l1'] + [f'rgb.l{i}' for i in range(len(eff) - 2)]
-        self._eff = (names, [(dW, db) for _, dW, db in eff], inv)
+        self._eff = (names, [(dW, db, segs, lin.weight_v.shape[1]) for lin, dW, db, segs in eff], inv)
         sink = _GradSink()
-        ents = [_wn_entry(sink, dW, db, bias=lin.bias, v=lin.weight_v, g=lin.weight_g) for lin, dW, db in eff]
+        ents = [_wn_entry(sink, dW, db, bias=lin.bias, v=lin.weight_v, g=lin.weight_g, segs=segs)
+                for lin, dW, db, segs in eff]
         head = sdf.mlp.linear_sdf
         ents.append(_wn_entry(sink, self.ws['d_whead'], self.ws['d_bhead'], weight=head.weight, bias=head.bias))
         ents.append(_wn_entry(sink, self.ws['d_s_var'].reshape(1, 1), weight=m.s_var))
@@ -973,7 +1000,7 @@ class FusedField:
             ents.append(_wn_entry(sink, g['app'], weight=m.appear_embed.weight))
         if self.bg:
             ents += self._scatter_background(g['bg'], inv, sink)
-        _weightnorm_bwd(ents, inv, dW0.device)
+        _weightnorm_bwd(ents, inv, gx.device, self._scal[4:5] if self.dynamic else None)
         if not self._table_in_place:
             _acc(sdf.tcnn_encoding.params, g['table'].to(sdf.tcnn_encoding.params.dtype))
 
@@ -981,7 +1008,8 @@ class FusedField:
     def eff_grads(self):
         """Unscaled gradients of the effective weights and biases of the last step, per layer."""
         names, eff, inv = self._eff
-        return {n: (dW * inv, db * inv) for n, (dW, db) in zip(names, eff)}
+        return {n: ((_mapped(dW, cols, segs) if segs else dW) * inv, db * inv)
+                for n, (dW, db, segs, cols) in zip(names, eff)}
 
     def _scatter_background(self, g, inv, sink):
         """Background NeRF gradients (plain linears) from the packed layouts: entries of the
@@ -1041,14 +1069,9 @@ class FusedField:
         self._scal[2].fill_(float(m.w_curv or 0.0))
 
     def _check_and_update_scale(self, scal):
-        """found_inf |= any non-finite master gradient (the scatter already flagged the table's);
-        then the scale update of GradScaler.update: x 0.5 on overflow, x 2 after growth_interval
-        clean steps in a row.  Device work only, no host synchronisation."""
-        table = self.model.neural_sdf.tcnn_encoding.params
-        small = [p.grad for p in self.model.parameters()
-                 if p.grad is not None and p is not table and p.grad.dtype == torch.float32]
-        if small:
-            torch._amp_foreach_non_finite_check_and_unscale_(small, scal[4:5], self._one)
+        """The scale update of GradScaler.update: x 0.5 on overflow, x 2 after growth_interval
+        clean steps in a row.  The scatter and the weight-norm backward have set found_inf if any
+        gradient they wrote is not finite.  Device work only, no host synchronisation."""
         torch._amp_update_scale_(scal[0:1], self._growth, scal[4:5], 2.0, 0.5, self.growth_interval)
 
     def found_inf(self):
@@ -1134,11 +1157,7 @@ class CapturedStep:
         table = model.neural_sdf.tcnn_encoding.params
         n_act = active_table_params(model.neural_sdf)
         with torch.cuda.graph(self.graph):
-            for p in self.params:
-                if p is table:
-                    p.grad[:n_act].zero_()
-                else:
-                    p.grad.zero_()
+            torch._foreach_zero_([p.grad[:n_act] if p is table else p.grad for p in self.params])
             self.out = fused.step(self.static, compute_loss=False, _refresh=False)
 
     def replay(self, batch=None):

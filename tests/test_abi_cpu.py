@@ -184,3 +184,23 @@ def test_weightnorm_pack_arguments_without_gpu(lib):
     assert b"no destination" in lib.gbsdf_last_error()
     assert lib.gbsdf_weightnorm_fwd(fused.WN_MAX_LAYERS + 1, None, None) == 1
     assert lib.gbsdf_weightnorm_fwd(0, None, None) == 0
+
+
+def test_weightnorm_map_layout_and_segment_checks():
+    """gbsdf_weightnorm_bwd_mapped: the binding's struct layout; segments outside the layer or the
+    gradient's rows are rejected before any launch."""
+    from neuralangelo_gb300 import fused
+    lib = _lib.load()
+    lib.gbsdf_weightnorm_map_size.restype = ctypes.c_size_t
+    assert lib.gbsdf_weightnorm_map_size() == ctypes.sizeof(fused.WeightNormMap)
+    one, ptr = ctypes.c_float(1.0), lambda a: ctypes.cast(a, ctypes.c_void_p)  # noqa: E731
+    layers, maps = (fused.WeightNormLayer * 1)(), (fused.WeightNormMap * 1)()
+    e, m = layers[0], maps[0]
+    e.rows, e.cols, e.dW, e.dv, e.ld_dw = 4, 8, 256, 256, 16
+    call = lambda: lib.gbsdf_weightnorm_bwd_mapped(1, ptr(layers), ptr(maps), None, one, None, None)  # noqa: E731
+    m.nseg = fused.WN_MAX_SEGMENTS + 1
+    assert call() == 1
+    m.nseg = 1
+    for dst, n, src, src2 in ((6, 3, 0, -1), (0, 8, 9, -1), (0, 8, 0, 9), (-1, 2, 0, -1), (0, 2, -1, -1)):
+        m.dst[0], m.n[0], m.src[0], m.src2[0] = dst, n, src, src2
+        assert call() == 1

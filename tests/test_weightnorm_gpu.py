@@ -206,3 +206,38 @@ def test_step_pack_matches_torch(background):
         with torch.no_grad():                   # the next pack must see updated masters
             for prm in model.parameters():
                 prm.add_(0.01 * torch.randn_like(prm))
+
+
+@pytest.mark.parametrize("acc", [False, True])
+def test_mapped_gradients_equal_the_assembled_ones(acc):
+    """Column segments (moved, summed, absent) read in place give bit for bit what the assembled
+    gradient gives, and a non-finite value written sets the flag."""
+    g = torch.Generator(DEV).manual_seed(3)
+    rows, cols = 37, 131
+    gx = torch.randn(rows, 160, device=DEV, generator=g)
+    segs = [(0, 3, 64, 68), (3, 64, 0, 80), (70, 61, 99, -1)]
+    got = []
+    for mapped in (False, True):
+        q = torch.Generator(DEV).manual_seed(4)
+        lin = torch.nn.Module()
+        lin.v = torch.nn.Parameter(torch.randn(rows, cols, device=DEV, generator=q))
+        lin.g = torch.nn.Parameter(torch.rand(rows, 1, device=DEV, generator=q) + 0.5)
+        lin.b = torch.nn.Parameter(torch.zeros(rows, device=DEV))
+        plain = torch.nn.Parameter(torch.zeros(rows, cols, device=DEV))
+        if acc:
+            for p in (lin.v, lin.g, lin.b, plain):
+                p.grad = torch.randn(p.shape, device=DEV, generator=q)
+        sink = fused._GradSink()
+        dW = gx if mapped else fused._mapped(gx, cols, segs)
+        kw = dict(segs=segs) if mapped else {}
+        flag = torch.zeros(1, device=DEV)
+        ents = [fused._wn_entry(sink, dW, gx[:, 67], bias=lin.b, v=lin.v, g=lin.g, **kw),
+                fused._wn_entry(sink, dW, weight=plain, **kw)]
+        fused._weightnorm_bwd(ents, 0.37, DEV, flag)
+        got.append([lin.v.grad, lin.g.grad, lin.b.grad, plain.grad])
+        assert flag.item() == 0
+    for a, b in zip(*got):
+        assert torch.equal(a, b)
+    gx[rows - 1, 159] = float("inf")
+    fused._weightnorm_bwd([fused._wn_entry(fused._GradSink(), gx, weight=plain, segs=segs)], 0.37, DEV, flag)
+    assert flag.item() == 1
