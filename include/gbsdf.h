@@ -521,6 +521,27 @@ int gbsdf_weightnorm_bwd_mapped(int32_t n, const gbsdf_weightnorm_layer* layers,
                                 const float* scale_dev, float scale, float* found_inf, void* stream);
 size_t gbsdf_weightnorm_map_size(void);
 
+/* A chain of dense layers in one launch, each layer's output handed to the next on chip as an fp16
+ * hi + lo pair (2 to GBSDF_MLP_MAX_LAYERS layers):  y_l = epi_l([y_{l-1} | in_l] W_l^T + bias_l), W_l [N, N_{l-1} + K_in] fp16
+ * row-major contiguous (the previous layer's columns first; the first layer has only in_l).
+ * Same products, order of accumulation and roundings as gbsdf_dense called layer by layer with
+ * both halves.  N 128 or 256, K_in % 16 == 0, at most 256 for the first and 128 for a later
+ * layer; in_hi / in_lo [M, ld_in] fp16 with K_in > 0; out_hi / out_lo [M, ld_out] fp16 receive the layer's halves, or NULL.  epi 0 identity,
+ * 1 relu, 2 softplus(beta).  Row strides multiples of 8, bases 16-byte aligned. */
+#define GBSDF_MLP_MAX_LAYERS 10
+typedef struct gbsdf_mlp_layer {
+    int32_t K_in, N, epi, ld_in;
+    const void* W;
+    const float* bias;        /* [N] or NULL */
+    const void* in_hi;
+    const void* in_lo;
+    void* out_hi;
+    void* out_lo;
+    int32_t ld_out, pad;
+} gbsdf_mlp_layer;
+int gbsdf_mlp_chain(int64_t M, int32_t n_layers, const gbsdf_mlp_layer* layers, float beta, int* err, void* stream);
+size_t gbsdf_mlp_layer_size(void);
+
 /* Working copies of weight-normalised (or plain) weights for the fused step: per entry, rows of
  * W = g v / ||v|| (the norm over all `cols` of each source row; g == NULL: W = v), columns
  * [col0, col0 + ncols), written to any of: dst16 (fp16, row stride ld16, the segment's first

@@ -18,7 +18,7 @@ device flag (``found_inf``) and halves the scale, and growth_interval clean step
 a row double it; the update runs on the device, inside a captured graph too.
 
 Kernels per step (all on the current stream):
-  field_fwd, dense x (1 + colour layers), rgb_head_fwd, render_fused,
+  field_fwd, mlp_chain (SDF feature layer and colour layers), rgb_head_fwd, render_fused,
   rgb_head_bwd (with the colour head's weight gradient), dense x (colour layers + 2),
   app_grad, field_bwd, and the weight gradients (tcgen05, fp16 in / fp32 out).
 """
@@ -130,6 +130,44 @@ def _wgrad(dZ, X, N, K, dW, accumulate=False, dZ_lo=None, err=None):
     _lib.call("gbsdf_wgrad", dZ.shape[0], N, K, c_vp(dZ.data_ptr()), c_vp(_p(dZ_lo)), dZ.stride(0),
               c_vp(X.data_ptr()), X.stride(0), c_vp(dW.data_ptr()), dW.stride(0), 1 if accumulate else 0,
               c_vp(_p(err)), _lib.stream_ptr(dZ.device))
+
+
+class MlpLayer(ctypes.Structure):
+    """gbsdf_mlp_layer (include/gbsdf.h)."""
+    _fields_ = [("K_in", c_i32), ("N", c_i32), ("epi", c_i32), ("ld_in", c_i32), ("W", c_vp), ("bias", c_vp),
+                ("in_hi", c_vp), ("in_lo", c_vp), ("out_hi", c_vp), ("out_lo", c_vp), ("ld_out", c_i32), ("pad", c_i32)]
+
+
+MLP_MAX_LAYERS = 10
+_lib.register("gbsdf_mlp_chain", [c_i64, c_i32, c_vp, c_f32, c_vp, c_vp])
+
+
+def _mlp_chain(layers, beta, err):
+    """gbsdf_mlp_chain: the layers (W, bias, epi, inp, out, out_lo) in one launch.  inp = (hi, lo, K)
+    are columns from global memory (all of the first layer's; appended ones later), out / out_lo
+    the fp16 buffers that receive the layer's halves, or None."""
+    arr = (MlpLayer * len(layers))()
+    first = layers[0][3][0]
+    M, moved = first.shape[0], 0
+    for y, (W, bias, epi, inp, out, out_lo) in zip(arr, layers):
+        assert W.is_contiguous()
+        y.N, y.epi, y.W, y.bias = W.shape[0], int(epi), W.data_ptr(), _p(bias)
+        if inp is not None:
+            hi, lo, y.K_in = inp
+            assert hi.stride(0) == lo.stride(0)
+            y.in_hi, y.in_lo, y.ld_in = hi.data_ptr(), lo.data_ptr(), hi.stride(0)
+            moved += 4 * y.K_in
+        y.out_hi, y.out_lo = _p(out), _p(out_lo)
+        if out is not None:
+            y.ld_out = out.stride(0)
+            moved += 2 * y.N
+        if out_lo is not None:
+            assert y.ld_out in (0, out_lo.stride(0))
+            y.ld_out = out_lo.stride(0)
+            moved += 2 * y.N
+    _lib.TIMER.count_bytes("gbsdf_mlp_chain", M * moved)
+    _lib.call("gbsdf_mlp_chain", M, len(layers), ctypes.cast(arr, c_vp), float(beta), c_vp(_p(err)),
+              _lib.stream_ptr(first.device))
 
 
 class WeightNormLayer(ctypes.Structure):
@@ -429,6 +467,9 @@ class FusedField:
             self.n_bg = int(cb.samples)
             self.Hbr = int(mb.hidden_dim_rgb)
             self.Kr0 = 256 + _round16(16 + self.app_dim + 1)   # [feat | SH 16, app, 1 | 0]
+        # activation pairs stay on chip between the forward layers (one launch for the feature
+        # layer and the colour MLP)
+        self.chain = self.pairs and 1 + self.n_rgb_hidden <= MLP_MAX_LAYERS
         self.ws = None
         self.err = None
         self._table16 = None          # persistent fp16 working copy of an FP32 table
@@ -603,8 +644,9 @@ class FusedField:
                                if self.deterministic else None))
         if self.pairs:
             # low halves, with the row strides of their hi buffers (the constant-1 column's lo is 0)
-            ws.update(h0c_lo=e(Ns, 264, dt=f16).zero_(), xc_lo=e(Ns, self.Kc0, dt=f16),
-                      ys_lo=[e(Ns, Hc + 8, dt=f16) for _ in range(self.n_rgb_hidden - 1)])
+            # (a chained forward reads only the field's own: h0c_lo, and the tail columns of xc_lo)
+            ws.update(h0c_lo=e(Ns, 264, dt=f16), xc_lo=e(Ns, self.Kc0, dt=f16),
+                      ys_lo=[None if self.chain else e(Ns, Hc + 8, dt=f16) for _ in range(self.n_rgb_hidden - 1)])
         else:
             ws.update(h0c_lo=None, xc_lo=None, ys_lo=[None] * (self.n_rgb_hidden - 1))
         if self.bg:
@@ -620,8 +662,10 @@ class FusedField:
                 # low halves of every background activation that feeds another layer's forward
                 # (or the density head); the colour hidden layer feeds the FP32 head only
                 z = lambda *sh: torch.zeros(*sh, device=device, dtype=f16)  # noqa: E731
-                ws.update(bg_S_lo=z(Nb, BG_S_COLS), bg_h_lo={i: z(Nb, 264) for i in (1, 2, 3, 5, 6, 7)},
-                          bg_G_lo=z(Nb, self.Kr0),
+                # (chained: the encoded columns, and layer 7's input for the density head)
+                ws.update(bg_S_lo=e(Nb, BG_S_COLS, dt=f16),
+                          bg_h_lo={i: None if self.chain and i != 7 else e(Nb, 264, dt=f16) for i in (1, 2, 3, 5, 6, 7)},
+                          bg_G_lo=e(Nb, self.Kr0, dt=f16),
                           # the backward's input gradients too: they pass through up to eight layers
                           # (the density column of dZ7 stays a single fp16 value: its lo is 0)
                           bg_dz_r_lo=z(Nb, Hbr), bg_dZ7_lo=z(Nb, 272), bg_dz_lo=[z(Nb, 256) for _ in range(2)])
@@ -728,17 +772,28 @@ class FusedField:
         # ---------------- forward ----------------
         _lib.call("gbsdf_field_encode", ctypes.byref(fa), stream)     # = gbsdf_field_fwd in two calls
         _lib.call("gbsdf_field_mlp_fwd", ctypes.byref(fa), stream)
-        # SDF feature layer, written into the colour input's first 256 columns
-        _dense(ws['h0c'], pk['w1'], 256, 256, ws['xc'], bias=pk['b1'], epi=EPI_SOFTPLUS, beta=fa.beta,
-               err=ws['err'], X_lo=ws['h0c_lo'], out_lo=ws['xc_lo'])
-        X, Xl, K = ws['xc'], ws['xc_lo'], self.Kc0
         n_last = self.n_rgb_hidden - 1
-        for i in range(self.n_rgb_hidden):
-            # the last hidden layer feeds only the FP32 colour head: single fp16 storage suffices
-            Yl = ws['ys_lo'][i] if i < n_last else None
-            _dense(X, pk['wc'][i], Hc, K, ws['ys'][i], bias=pk['bc'][i], epi=EPI_RELU, err=ws['err'], X_lo=Xl,
-                   out_lo=Yl)
-            X, Xl, K = ws['ys'][i], Yl, Hc
+        if self.chain:
+            # SDF feature layer (into the colour input's first 256 columns) and the colour MLP's hidden
+            # layers; the backward reads every layer's hi half, an evaluation only the last one's
+            keep = not _evaluate
+            tail = (ws['xc'][:, 256:], ws['xc_lo'][:, 256:], self.Kc0 - 256)
+            layers = [(pk['w1'], pk['b1'], EPI_SOFTPLUS, (ws['h0c'], ws['h0c_lo'], 256), ws['xc'] if keep else None, None)]
+            for i in range(self.n_rgb_hidden):
+                layers.append((pk['wc'][i], pk['bc'][i], EPI_RELU, tail if i == 0 else None,
+                               ws['ys'][i] if keep or i == n_last else None, None))
+            _mlp_chain(layers, fa.beta, ws['err'])
+        else:
+            # SDF feature layer, written into the colour input's first 256 columns
+            _dense(ws['h0c'], pk['w1'], 256, 256, ws['xc'], bias=pk['b1'], epi=EPI_SOFTPLUS, beta=fa.beta,
+                   err=ws['err'], X_lo=ws['h0c_lo'], out_lo=ws['xc_lo'])
+            X, Xl, K = ws['xc'], ws['xc_lo'], self.Kc0
+            for i in range(self.n_rgb_hidden):
+                # the last hidden layer feeds only the FP32 colour head: single fp16 storage suffices
+                Yl = ws['ys_lo'][i] if i < n_last else None
+                _dense(X, pk['wc'][i], Hc, K, ws['ys'][i], bias=pk['bc'][i], epi=EPI_RELU, err=ws['err'], X_lo=Xl,
+                       out_lo=Yl)
+                X, Xl, K = ws['ys'][i], Yl, Hc
         ylast = ws['ys'][-1]
         _lib.TIMER.count_bytes("gbsdf_rgb_head_fwd", Ns * (Hc * 2 + 12))
         _lib.call("gbsdf_rgb_head_fwd", Ns, c_vp(ylast.data_ptr()), ylast.stride(0), Hc, c_vp(pk['wl'].data_ptr()),
@@ -748,7 +803,7 @@ class FusedField:
             dists_bg = batch['dists_bg'].reshape(-1).contiguous().float()
             if dists_bg.numel() != R * self.n_bg:
                 raise ValueError(f"dists_bg must hold {self.n_bg} background samples per ray")
-            self._background_forward(R, center, ray_unit, dists_bg, app_idx, stream)
+            self._background_forward(R, center, ray_unit, dists_bg, app_idx, stream, keep=not _evaluate)
         # ---------------- render + losses, fwd + bwd ----------------
         lw = m.cfg.loss_weight
         n_mean = batch.get('mean_count', Ns)
@@ -868,7 +923,7 @@ class FusedField:
         return out
 
     # ------------------------------------------------------------------ background NeRF
-    def _background_forward(self, R, center, ray_unit, dists_bg, app_idx, stream):
+    def _background_forward(self, R, center, ray_unit, dists_bg, app_idx, stream, keep=True):
         """BackgroundNeRF.forward (modules.py:268-284) of the R x n_bg background samples:
         encode -> 8 ReLU layers with the input concatenated at layer 4 -> density head and
         256 features -> [features, SH(d), app] -> ReLU -> sigmoid colour."""
@@ -886,21 +941,33 @@ class FusedField:
                   G.stride(0), Kr0 - 256, stream)
         err = ws['err']
         w, b = pk['bw'], pk['bb']
-        _dense(X, w[0], 256, BG_X_COLS, h[1], bias=b[0], epi=EPI_RELU, err=err, X_lo=Xl, out_lo=hl[1])
-        _dense(h[1], w[1], 256, 256, h[2], bias=b[1], epi=EPI_RELU, err=err, X_lo=hl[1], out_lo=hl[2])
-        _dense(h[2], w[2], 256, 256, h[3], bias=b[2], epi=EPI_RELU, err=err, X_lo=hl[2], out_lo=hl[3])
-        _dense(h[3], w[3], 256, 256, S, bias=b[3], epi=EPI_RELU, err=err,             # h4 into S[:, :256]
-               X_lo=hl[3], out_lo=Sl)
-        _dense(S, w[4], 256, BG_S_COLS, h[5], bias=b[4], epi=EPI_RELU, err=err,       # skip: [h4 | input]
-               X_lo=Sl, out_lo=hl[5])
-        _dense(h[5], w[5], 256, 256, h[6], bias=b[5], epi=EPI_RELU, err=err, X_lo=hl[5], out_lo=hl[6])
-        _dense(h[6], w[6], 256, 256, h[7], bias=b[6], epi=EPI_RELU, err=err, X_lo=hl[6], out_lo=hl[7])
-        _dense(h[7], w[7], 256, 256, G, bias=b[7], epi=EPI_RELU, err=err,             # features into G[:, :256]
-               X_lo=hl[7], out_lo=Gl)
+        hr = ws['bg_hr']
+        enc, tail = (X, Xl, BG_X_COLS), (Gt, Gtl, Kr0 - 256)
+        head = self.chain and Hbr >= 128                 # the colour layer's width fits the chain
+        if self.chain:
+            o = (lambda t: t) if keep else (lambda t: None)   # noqa: E731  (hi halves that only the backward reads)
+            outs = [o(h[1]), o(h[2]), o(h[3]), o(S), o(h[5]), o(h[6]), h[7], o(G) if head else G]
+            los = [None] * 6 + [hl[7], None if head else Gl]
+            layers = [(w[i], b[i], EPI_RELU, enc if i in (0, 4) else None, outs[i], los[i]) for i in range(8)]
+            if head:
+                layers.append((pk['bwr0'], pk['bbr0'], EPI_RELU, tail, hr, None))
+            _mlp_chain(layers, 1.0, err)
+        else:
+            _dense(X, w[0], 256, BG_X_COLS, h[1], bias=b[0], epi=EPI_RELU, err=err, X_lo=Xl, out_lo=hl[1])
+            _dense(h[1], w[1], 256, 256, h[2], bias=b[1], epi=EPI_RELU, err=err, X_lo=hl[1], out_lo=hl[2])
+            _dense(h[2], w[2], 256, 256, h[3], bias=b[2], epi=EPI_RELU, err=err, X_lo=hl[2], out_lo=hl[3])
+            _dense(h[3], w[3], 256, 256, S, bias=b[3], epi=EPI_RELU, err=err,             # h4 into S[:, :256]
+                   X_lo=hl[3], out_lo=Sl)
+            _dense(S, w[4], 256, BG_S_COLS, h[5], bias=b[4], epi=EPI_RELU, err=err,       # skip: [h4 | input]
+                   X_lo=Sl, out_lo=hl[5])
+            _dense(h[5], w[5], 256, 256, h[6], bias=b[5], epi=EPI_RELU, err=err, X_lo=hl[5], out_lo=hl[6])
+            _dense(h[6], w[6], 256, 256, h[7], bias=b[6], epi=EPI_RELU, err=err, X_lo=hl[6], out_lo=hl[7])
+            _dense(h[7], w[7], 256, 256, G, bias=b[7], epi=EPI_RELU, err=err,             # features into G[:, :256]
+                   X_lo=hl[7], out_lo=Gl)
         _lib.call("gbsdf_bg_density", Nb, c_vp(h[7].data_ptr()), c_vp(_p(hl[7])), h[7].stride(0), 256,
                   c_vp(pk['bw7d'].data_ptr()), c_vp(pk['bb7d'].data_ptr()), c_vp(ws['bg_sigma'].data_ptr()), stream)
-        hr = ws['bg_hr']
-        _dense(G, pk['bwr0'], Hbr, Kr0, hr, bias=pk['bbr0'], epi=EPI_RELU, err=err, X_lo=Gl)
+        if not head:
+            _dense(G, pk['bwr0'], Hbr, Kr0, hr, bias=pk['bbr0'], epi=EPI_RELU, err=err, X_lo=Gl)
         _lib.call("gbsdf_rgb_head_fwd", Nb, c_vp(hr.data_ptr()), hr.stride(0), Hbr, c_vp(pk['bwr1'].data_ptr()),
                   c_vp(pk['bbr1'].data_ptr()), c_vp(ws['bg_rgbs'].data_ptr()), stream)
 
