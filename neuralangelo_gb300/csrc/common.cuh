@@ -198,6 +198,28 @@ __device__ __forceinline__ float warp_column_sum16(float* v, int lane) {
     return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 16);
 }
 
+// Adds v into row `entry` (8 floats, 16-byte aligned) of table for every lane with `on`; the whole
+// warp calls.  Neighbouring lanes trade halves first, so that each of the two vector atomics
+// covers whole 32-byte rows of every other lane: with one row per lane in both, each touched 32 half
+// sectors, twice the requests at L1 and L2.
+__device__ __forceinline__ void scatter_add_rows8(float* table, uint64_t entry, bool on, const float* v, int lane) {
+    const bool odd = lane & 1;
+    float a[4], b[4];                       // this lane's half of the even and of the odd lane's row
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const float got = __shfl_xor_sync(0xffffffffu, odd ? v[k] : v[4 + k], 1);
+        a[k] = odd ? got : v[k];
+        b[k] = odd ? v[4 + k] : got;
+    }
+    const uint64_t other = __shfl_xor_sync(0xffffffffu, (unsigned long long)entry, 1);
+    const unsigned both = __ballot_sync(0xffffffffu, on);
+    float* half = table + (odd ? 4 : 0);
+    if ((both >> (lane & ~1)) & 1u)
+        atomicAdd(reinterpret_cast<float4*>(half + (odd ? other : entry) * 8), make_float4(a[0], a[1], a[2], a[3]));
+    if ((both >> (lane | 1)) & 1u)
+        atomicAdd(reinterpret_cast<float4*>(half + (odd ? entry : other) * 8), make_float4(b[0], b[1], b[2], b[3]));
+}
+
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);

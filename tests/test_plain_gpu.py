@@ -139,3 +139,46 @@ def test_plain_model_matches_golden(name):
     for k in z:
         if k.startswith('g_sdf.') or k.startswith('g_rgb.'):
             assert rel(grads[k[2:]], z[k]) < 1e-3, k
+
+
+@pytest.mark.parametrize("F", [1, 2, 4, 8])
+@pytest.mark.parametrize("M", [1, 31, 257])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_hashgrid_rows_at_every_alignment(F, M, shift):
+    """Rows as vectors and, ``shift`` elements off, element by element, both table and output types;
+    a backward whose warps are partly empty or carry zero rows."""
+    import ctypes
+    from neuralangelo_gb300 import _lib
+    from neuralangelo_gb300.encoding import GridLayout
+    from oracle import hashgrid as hg
+    lay, ora = GridLayout(5, F, 9, 8, 1.7), hg.level_layout(5, F, 9, 8, 1.7)
+    g = torch.Generator().manual_seed(F * 100 + M)
+    x = torch.rand(M, 3, generator=g)
+    xd = x.to(DEV)
+    stream = _lib.stream_ptr(xd.device)
+    tab = torch.randn(lay.n_params, generator=g).half().float()
+    want = hg.encode(x.numpy(), tab.double().numpy(), ora, 4)
+    scale = float(tab.abs().max())
+    for tdt, tt in ((_lib.F32, torch.float32), (_lib.F16, torch.float16)):
+        # (the entry point wants a 16-byte aligned table)
+        off = 4 * shift if tt == torch.float32 else 8 * shift
+        t = torch.zeros(lay.n_params + 16, device=DEV, dtype=tt)[off:off + lay.n_params].copy_(tab)
+        for odt, ot in ((_lib.F32, torch.float32), (_lib.F16, torch.float16)):
+            buf = torch.full((M * 5 * F + 2,), 7.0, device=DEV, dtype=ot)
+            out = buf[shift:shift + M * 5 * F]
+            _lib.call("gbsdf_hashgrid_fwd", ctypes.byref(lay.struct), 4, _lib.ptr(xd), M, ctypes.c_void_p(t.data_ptr()),
+                      tdt, ctypes.c_void_p(out.data_ptr()), odt, stream)
+            tol = scale * 16 * 2.0 ** -24 + (scale * 2.0 ** -11 if ot == torch.float16 else 0)
+            assert np.abs(out.double().cpu().numpy().reshape(M, -1) - want).max() <= tol
+            assert bool((buf[:shift] == 7).all()) and bool((buf[shift + M * 5 * F:] == 7).all())
+    d = torch.randn(M, 5 * F, generator=g)
+    d[::3] = 0
+    buf = torch.zeros(M * 5 * F + 2, device=DEV)
+    dd = buf[shift:shift + M * 5 * F].copy_(d.reshape(-1))
+    grad = torch.zeros(lay.n_params, device=DEV)
+    _lib.call("gbsdf_hashgrid_bwd", ctypes.byref(lay.struct), 4, _lib.ptr(xd), M, ctypes.c_void_p(dd.data_ptr()),
+              _lib.ptr(grad), stream)
+    ref = hg.encode_backward(x.numpy(), d.double().numpy(), ora, 4)
+    mag = hg.encode_backward(x.numpy(), d.double().abs().numpy(), ora, 4)
+    # float32 products and sums of at most 8 M terms in any order
+    assert (np.abs(grad.double().cpu().numpy().reshape(-1, F) - ref) <= mag * (8 * M + 8) * 2.0 ** -24).all()
