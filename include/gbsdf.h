@@ -233,7 +233,7 @@ typedef struct gbsdf_field_args {
                                          give bit-identical table gradients (|sum| < 2^15).  The call
                                          clears the buffer itself.  NULL: FP32 vector atomics. */
     /* Launch shapes (tuning choices, results unchanged; 0 = the built-in default): */
-    int32_t scatter_cpt;     /* table corners per pass of the scatter for 8-feature fields: 2, 4 or 8 */
+    int32_t scatter_cpt;     /* samples per thread of the scatter: 2, 4 or 8 for one, two or four (0 = by size) */
     int32_t fwd_ctas;        /* CTAs per SM launched for the MLP forward: 1 or 2 */
 } gbsdf_field_args;
 

@@ -387,20 +387,20 @@ __global__ void __launch_bounds__(GATHER_THREADS, 4) k_field_gather(FieldParams 
     }
 }
 
-// Table gradient of one (sample, level) over the sample's 7 evaluations.  The thread owns the
-// eight corners of the centre's cell: an evaluation in that cell adds to all eight, one in a
+// Table gradient of one level over NS consecutive samples and their evaluations.  The thread owns
+// the eight corners of the centre's cell: an evaluation in that cell adds to all eight, one in a
 // neighbouring cell to the corners the two cells share (its weight at a shared corner is a
-// product of one factor per axis, zero for the corners it does not reach), so each owned corner
-// leaves as one vector atomic.  The corners of neighbouring cells that the centre's cell does
-// not have (typically four per evaluation, of about one evaluation in nine) go out directly,
-// the evaluations packed across the warp so that they cost one or two dense passes.
-// Merging only consecutive evaluations of equal cells instead flushed a corner again after
-// every tap that left the cell: about 1.8 times the atomics (L1 at 90 %, L2 atomics at 69 %).
-// The corners go in passes of CPT (the positions and d_enc rows are read again per pass, from
-// L1): fewer accumulator registers, more resident warps.
-// 2.1 M samples x 8 levels took 3.05 ms in the consecutive form and take 2.28 ms (2.62 ms
-// with 2 corners per pass, 2.47 ms with 8); 0.24 M samples x 16 levels 0.99 and 0.72 ms.
-constexpr int SCATTER_CPT = 4;
+// product of one factor per axis, zero for the corners it does not reach).  While the next sample's
+// centre stays in the cell, as it mostly does at coarse levels, the sums go on in registers; then
+// each owned corner leaves as one vector atomic.  The corners of neighbouring cells that the
+// centre's cell does not have (typically four per evaluation, of about one evaluation in nine) go
+// out directly, the evaluations packed across the warp so that they cost a few dense passes.
+// Eight features are two lanes' work, four each: the accumulators fit the registers in one pass,
+// and the pair's atomics cover whole 32-byte rows.
+// 2.1 M samples x 8 levels: 3.05 ms merging consecutive evaluations of equal cells, 2.28 ms with the
+// corners owned over one sample (four per pass, all features in one lane, neighbouring samples
+// merged by shuffles), 2.09 ms so; 0.24 M samples x 16 levels: 0.99, 0.72 and 0.50 ms (there the half
+// sectors of 16-byte atomics counted).  Evaluations not unrolled 2.38 ms, two blocks per SM 2.55.
 constexpr int SCATTER_THREADS = 256;
 
 // d_enc of one evaluation and level
@@ -425,134 +425,148 @@ __device__ __forceinline__ bool any_nonfinite(const float* g) {
     return bad;
 }
 
-template <int F, int CPT, int TAPS, bool DET>
-__global__ void __launch_bounds__(SCATTER_THREADS, CPT >= 8 ? 2 : (CPT == 4 ? 3 : 4)) k_field_scatter(FieldParams p) {
+template <int F, int TAPS, bool DET, int NS>
+__global__ void __launch_bounds__(SCATTER_THREADS, 3) k_field_scatter(FieldParams p) {
     constexpr int EVALS = TapTile<TAPS>::EVALS, SPT = TapTile<TAPS>::SPT;
+    constexpr int FS = F < 4 ? F : 4, PARTS = F / FS;     // features per lane, lanes per (samples, level)
     __shared__ LevelDesc lv_s[GBSDF_MAX_LEVELS];
-    __shared__ uint8_t list_s[SCATTER_THREADS / 32][32 * TAPS];
+    __shared__ uint16_t list_s[SCATTER_THREADS / 32][32 / PARTS * NS * TAPS];
     const int A = p.active, K0 = p.K0;
     stage_levels(p.grid, lv_s, A);
     __syncthreads();
     // 32-bit index arithmetic: the launcher checks Ns * active * 8 < 2^32
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool in = i < (uint32_t)p.Ns * (uint32_t)A;     // (whole warps go on: they merge and pack together)
-    const uint32_t s32 = in ? i / (uint32_t)A : 0u;
-    const int l = in ? (int)(i - s32 * (uint32_t)A) : 0;
-    const uint32_t t = s32 / SPT;
-    const uint32_t row0 = t * (SPT * EVALS) + (s32 - t * SPT);   // evaluation e's row: row0 + e * SPT
-    const int lane = threadIdx.x & 31;
+    const int part = (int)(i % PARTS), lane = threadIdx.x & 31;
+    const uint32_t item = i / PARTS, group = item / (uint32_t)A;
+    const int l = (int)(item - group * (uint32_t)A);
+    const uint32_t s0 = group * NS;
+    const uint32_t n = s0 < (uint32_t)p.Ns ? min((uint32_t)p.Ns - s0, (uint32_t)NS) : 0u;   // (whole warps go on)
     const float gscale = p.d_table_scale_dev ? *p.d_table_scale_dev : (p.d_table_scale != 0.0f ? p.d_table_scale : 1.0f);
     auto add = [&](uint64_t entry, const float* v) {
-        if constexpr (DET) scatter_add_fixed<F>(p.d_table_fix + entry * F, v);
-        else scatter_add<F>(p.d_table + entry * F, v);
+        if constexpr (DET) scatter_add_fixed<FS>(p.d_table_fix + entry * F + part * FS, v);
+        else scatter_add<FS>(p.d_table + entry * F + part * FS, v);
     };
-    // With a power of two of active levels the lanes l, l + A, l + 2A, .. of a warp hold level l
-    // of consecutive samples, which at coarse levels often sit in the same cell.  Xor-shuffle
-    // steps merge equal entries: two lanes merge only when both still own their sums, the
-    // lower lane absorbing the upper one's, so every contribution is written exactly once.
-    const bool grouped = (A & (A - 1)) == 0;
+    // (first row of sample s; evaluation e's is e * SPT rows on)
+    auto row_of = [](uint32_t s) {
+        const uint32_t t = s / SPT;
+        return t * (SPT * EVALS) + (s - t * SPT);
+    };
     bool nonfinite = false;
-    uint32_t mask = 0;                                    // evaluations outside the centre's cell
-    float c[3] = {0.f, 0.f, 0.f};
-    if (in) sample_point(p, s32, c);
-    const LevelDesc d = lv_s[l];
-    const GridCell g0 = grid_cell(d.scale, c);
-#pragma unroll 1
-    for (int c0 = 0; c0 < 8; c0 += CPT) {
-        float acc[CPT][F];
+    uint32_t mask[NS];                                    // per sample: evaluations outside the centre's cell
+    const LevelDesc d = lv_s[n > 0 ? l : 0];
+    uint32_t home[3] = {0, 0, 0};
+    float acc[8][FS];
+    auto flush = [&]() {
 #pragma unroll
-        for (int cc = 0; cc < CPT; ++cc)
+        for (int c = 0; c < 8; ++c) {
+            add(d.offset + grid_index(d, home[0] + (c & 1), home[1] + ((c >> 1) & 1), home[2] + ((c >> 2) & 1)), acc[c]);
 #pragma unroll
-            for (int f = 0; f < F; ++f) acc[cc][f] = 0.0f;
+            for (int f = 0; f < FS; ++f) acc[c][f] = 0.0f;
+        }
+    };
+#pragma unroll
+    for (int c = 0; c < 8; ++c)
+#pragma unroll
+        for (int f = 0; f < FS; ++f) acc[c][f] = 0.0f;
 #pragma unroll 1
-        for (int e = 0; in && e < EVALS; ++e) {
-            float x[3], g[F];
-            load_d_enc<F>(p.d_enc + (int64_t)(row0 + e * SPT) * K0 + l * F, g);
+    for (uint32_t k = 0; k < n; ++k) {
+        float c[3];
+        sample_point(p, s0 + k, c);
+        const GridCell g0 = grid_cell(d.scale, c);
+        if (k > 0 && (g0.b[0] != home[0] || g0.b[1] != home[1] || g0.b[2] != home[2])) flush();
+#pragma unroll
+        for (int x = 0; x < 3; ++x) home[x] = g0.b[x];
+        const float* dv = p.d_enc + (int64_t)row_of(s0 + k) * K0 + l * F + part * FS;
+        uint32_t m = 0;
+#pragma unroll
+        for (int e = 0; e < EVALS; ++e) {
+            float x[3], g[FS];
+            load_d_enc<FS>(dv + (int64_t)e * SPT * K0, g);
             eval_point<TAPS>(c, e, p.eps, x);
             const GridCell gc = grid_cell(d.scale, x);
             // per axis: the weight of the owned corners at 0 and 1
             float w0[3], w1[3];
             bool other = false;
 #pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                const int db = (int)(gc.b[k] - g0.b[k]);
-                const float one_f = __fsub_rn(1.0f, gc.f[k]);
-                w0[k] = db == 0 ? one_f : (db == -1 ? gc.f[k] : 0.0f);
-                w1[k] = db == 0 ? gc.f[k] : (db == 1 ? one_f : 0.0f);
+            for (int a = 0; a < 3; ++a) {
+                const int db = (int)(gc.b[a] - home[a]);
+                const float one_f = __fsub_rn(1.0f, gc.f[a]);
+                w0[a] = db == 0 ? one_f : (db == -1 ? gc.f[a] : 0.0f);
+                w1[a] = db == 0 ? gc.f[a] : (db == 1 ? one_f : 0.0f);
                 other |= db != 0;
             }
-            const bool bad = any_nonfinite<F>(g);
+            const bool bad = any_nonfinite<FS>(g);
             nonfinite |= bad;
-            if (other) mask |= 1u << e;
+            if (other) m |= 1u << e;
             // (a non-finite gradient of another cell would reach every owned corner as 0 * inf:
             // that evaluation goes out corner by corner below)
             if (other && bad) continue;
 #pragma unroll
-            for (int cc = 0; cc < CPT; ++cc) {
-                const int corner = c0 + cc;
+            for (int f = 0; f < FS; ++f) g[f] *= gscale;
+#pragma unroll
+            for (int corner = 0; corner < 8; ++corner) {
                 const float wx = (corner & 1) ? w1[0] : w0[0], wy = (corner & 2) ? w1[1] : w0[1];
                 const float wz = (corner & 4) ? w1[2] : w0[2];
-                const float w = __fmul_rn(__fmul_rn(wx, wy), wz) * gscale;
+                const float w = __fmul_rn(__fmul_rn(wx, wy), wz);
 #pragma unroll
-                for (int f = 0; f < F; ++f) acc[cc][f] = fmaf(w, g[f], acc[cc][f]);
+                for (int f = 0; f < FS; ++f) acc[corner][f] = fmaf(w, g[f], acc[corner][f]);
             }
         }
 #pragma unroll
-        for (int cc = 0; cc < CPT; ++cc) {
-            const int corner = c0 + cc;
-            const uint32_t idx = grid_index(d, g0.b[0] + (corner & 1), g0.b[1] + ((corner >> 1) & 1),
-                                            g0.b[2] + ((corner >> 2) & 1));
-            bool mine = in;
-            if (grouped) {
-                for (int off = A; off <= 16; off <<= 1) {
-                    const uint32_t other_idx = __shfl_xor_sync(0xffffffffu, idx, off);
-                    const bool other_mine = __shfl_xor_sync(0xffffffffu, mine ? 1 : 0, off) != 0;
-                    float other[F];
-#pragma unroll
-                    for (int f = 0; f < F; ++f) other[f] = __shfl_xor_sync(0xffffffffu, acc[cc][f], off);
-                    if (mine && other_mine && other_idx == idx) {
-                        if ((lane & off) == 0) {
-#pragma unroll
-                            for (int f = 0; f < F; ++f) acc[cc][f] += other[f];
-                        } else {
-                            mine = false;
-                        }
-                    }
-                }
-            }
-            if (mine) add(d.offset + idx, acc[cc]);
-        }
+        for (int j = 0; j < NS; ++j)
+            if ((uint32_t)j == k) mask[j] = m;
     }
+    if (n > 0) flush();
     if (nonfinite && p.found_inf) *p.found_inf = 1.0f;     // any writer stores the same value
-    // the corners that the centre's cell does not have
-    uint8_t* list = list_s[threadIdx.x >> 5];
-    const int total = warp_pack_evals<EVALS>(mask, list, lane);
-    for (int k0 = 0; k0 < total; k0 += 32) {
-        const bool on = k0 + lane < total;
-        const int ent = on ? list[k0 + lane] : 0, own = ent >> 3, e = ent & 7;
-        const float oc[3] = {__shfl_sync(0xffffffffu, c[0], own), __shfl_sync(0xffffffffu, c[1], own),
-                             __shfl_sync(0xffffffffu, c[2], own)};
+    // the corners that the centre's cell does not have: (lane, sample, evaluation) entries of the first lane of
+    // each pair, taken by the pairs in turn
+    uint16_t* list = list_s[threadIdx.x >> 5];
+    int mine = 0;
+#pragma unroll
+    for (int j = 0; j < NS; ++j) {
+        if ((uint32_t)j >= n || part > 0) mask[j] = 0;
+        mine += __popc(mask[j]);
+    }
+    int at = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, at, o);
+        if (lane >= o) at += v;
+    }
+    const int total = __shfl_sync(0xffffffffu, at, 31);
+    at -= mine;
+#pragma unroll
+    for (int j = 0; j < NS; ++j)
+        for (uint32_t left = mask[j]; left; left &= left - 1)
+            list[at++] = (uint16_t)(lane << 8 | j << 4 | (__ffs(left) - 1));
+    __syncwarp();
+    for (int k0 = 0; k0 < total; k0 += 32 / PARTS) {
+        const int k = k0 + lane / PARTS;
+        const bool on = k < total;
+        const uint32_t ent = on ? list[k] : 0u;
+        const int own = (int)(ent >> 8), e = (int)(ent & 15u);
+        const uint32_t s = __shfl_sync(0xffffffffu, s0, own) + ((ent >> 4) & 15u);
         const int ol = __shfl_sync(0xffffffffu, l, own);
-        const uint32_t orow = __shfl_sync(0xffffffffu, row0, own);
         if (!on) continue;
-        float x[3], g[F];
-        load_d_enc<F>(p.d_enc + (int64_t)(orow + e * SPT) * K0 + ol * F, g);
-        eval_point<TAPS>(oc, e, p.eps, x);
+        float c[3], x[3], g[FS];
+        sample_point(p, s, c);
+        load_d_enc<FS>(p.d_enc + (int64_t)(row_of(s) + e * SPT) * K0 + ol * F + part * FS, g);
+        eval_point<TAPS>(c, e, p.eps, x);
         const LevelDesc od = lv_s[ol];
-        const GridCell home = grid_cell(od.scale, oc), gc = grid_cell(od.scale, x);
-        const bool bad = any_nonfinite<F>(g);
+        const GridCell centre = grid_cell(od.scale, c), gc = grid_cell(od.scale, x);
+        const bool bad = any_nonfinite<FS>(g);
         uint32_t db[3];
 #pragma unroll
-        for (int k = 0; k < 3; ++k) db[k] = gc.b[k] - home.b[k];
+        for (int a = 0; a < 3; ++a) db[a] = gc.b[a] - centre.b[a];
 #pragma unroll
         for (int corner = 0; corner < 8; ++corner) {
             const uint32_t bx = corner & 1, by = (corner >> 1) & 1, bz = (corner >> 2) & 1;
             // owned: the corner's coordinate relative to the centre's cell is 0 or 1 on every axis
             if (!bad && db[0] + bx <= 1u && db[1] + by <= 1u && db[2] + bz <= 1u) continue;
             const float w = corner_weight(corner, gc.f[0], gc.f[1], gc.f[2]) * gscale;
-            float v[F];
+            float v[FS];
 #pragma unroll
-            for (int f = 0; f < F; ++f) v[f] = w * g[f];
+            for (int f = 0; f < FS; ++f) v[f] = w * g[f];
             add(od.offset + grid_index(od, gc.b[0] + bx, gc.b[1] + by, gc.b[2] + bz), v);
         }
     }
@@ -1699,6 +1713,13 @@ static int x0ext_maps(const FieldParams& p, int64_t rows, int lo_cols, CUtensorM
                                     "x0ext lo");
 }
 
+template <int F, int TAPS, bool DET>
+static void launch_scatter(int ns, unsigned blocks, const FieldParams& p, cudaStream_t s) {
+    if (ns == 4) k_field_scatter<F, TAPS, DET, 4><<<blocks, SCATTER_THREADS, 0, s>>>(p);
+    else if (ns == 2) k_field_scatter<F, TAPS, DET, 2><<<blocks, SCATTER_THREADS, 0, s>>>(p);
+    else k_field_scatter<F, TAPS, DET, 1><<<blocks, SCATTER_THREADS, 0, s>>>(p);
+}
+
 template <int F, int TAPS>
 static int launch_field(const FieldParams& p, int which, cudaStream_t s) {
     constexpr int EVALS = TapTile<TAPS>::EVALS, SPT = TapTile<TAPS>::SPT, TILE_ROWS = TapTile<TAPS>::ROWS;
@@ -1810,8 +1831,16 @@ static int launch_field(const FieldParams& p, int which, cudaStream_t s) {
         if (int st = launch_status("field backward")) return st;
     }
     if (which & FK_SCATTER) {
-        const int64_t items = p.Ns * p.active;
-        const unsigned blocks = (unsigned)((items + SCATTER_THREADS - 1) / SCATTER_THREADS);
+        constexpr int PARTS = F < 4 ? 1 : F / 4;
+        // Samples per thread: four where that leaves two blocks' threads for every slot of the chip, fewer
+        // for small batches (2048 samples x 8 levels: 6.3 us with one, 20.1 with four; 2.1 M x 8: 2.53 ms
+        // with one, 2.31 with two, 2.09 with four, 2.21 with eight).
+        // p.scatter_cpt (a tuning choice): 2, 4 or 8 for one, two or four samples per thread
+        const int64_t slots = (int64_t)num_sms() * 3 * SCATTER_THREADS, lanes = p.Ns * p.active * PARTS;
+        int ns = lanes >= 8 * slots ? 4 : lanes >= 4 * slots ? 2 : 1;
+        if (p.scatter_cpt) ns = p.scatter_cpt / 2;
+        const int64_t threads = (p.Ns + ns - 1) / ns * p.active * PARTS;
+        const unsigned blocks = (unsigned)((threads + SCATTER_THREADS - 1) / SCATTER_THREADS);
         if (p.d_table_fix) {
             // deterministic mode: integer accumulation into the caller's buffer, then into d_table
             const int64_t n = (int64_t)p.grid.offset[p.grid.n_levels] * F;
@@ -1819,17 +1848,11 @@ static int launch_field(const FieldParams& p, int which, cudaStream_t s) {
                 set_error("clearing d_table_fix failed");
                 return GBSDF_ERR_CUDA;
             }
-            k_field_scatter<F, SCATTER_CPT, TAPS, true><<<blocks, SCATTER_THREADS, 0, s>>>(p);
+            launch_scatter<F, TAPS, true>(ns, blocks, p, s);
             if (int st = launch_status("field scatter (deterministic)")) return st;
             k_fixed_to_table<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(n, p.d_table_fix, p.d_table);
         } else {
-            // p.scatter_cpt (a tuning choice, 8-feature fields): table corners per pass, 2, 4 or 8
-            if (F == 8 && p.scatter_cpt == 2)
-                k_field_scatter<F, 2, TAPS, false><<<blocks, SCATTER_THREADS, 0, s>>>(p);
-            else if (F == 8 && p.scatter_cpt == 8)
-                k_field_scatter<F, 8, TAPS, false><<<blocks, SCATTER_THREADS, 0, s>>>(p);
-            else
-                k_field_scatter<F, SCATTER_CPT, TAPS, false><<<blocks, SCATTER_THREADS, 0, s>>>(p);
+            launch_scatter<F, TAPS, false>(ns, blocks, p, s);
         }
         if (int st = launch_status("field scatter")) return st;
     }
@@ -1850,7 +1873,7 @@ static int check_field(const FieldParams& p) {
     GBSDF_CHECK_ARG(p.Ns >= 0, "Ns < 0");
     GBSDF_CHECK_ARG(p.taps == 0 || p.taps == 4 || p.taps == 6, "taps %d (4 or 6; 0 means 6)", p.taps);
     GBSDF_CHECK_ARG(p.scatter_cpt == 0 || p.scatter_cpt == 2 || p.scatter_cpt == 4 || p.scatter_cpt == 8,
-                    "scatter_cpt %d (2, 4 or 8; 0 = 2)", p.scatter_cpt);
+                    "scatter_cpt %d (2, 4 or 8; 0 = by size)", p.scatter_cpt);
     GBSDF_CHECK_ARG(p.fwd_ctas >= 0 && p.fwd_ctas <= 2, "fwd_ctas %d (1 or 2; 0 = 2)", p.fwd_ctas);
     if (int st = check_field_weights(p)) return st;
     GBSDF_CHECK_ARG(p.S > 0 || p.sample_ray, "need S > 0 or sample_ray");
