@@ -164,6 +164,66 @@ __device__ __forceinline__ float softplus_fast_h(float z, const SoftplusK& k) {
     return t > k.tthr ? z : hl;
 }
 
+// Two float32 values in one register pair.  The packed operations round each as the single one does and
+// take half the issue slots.
+__device__ __forceinline__ uint64_t pack_f32x2(float lo, float hi) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void unpack_f32x2(uint64_t v, float& lo, float& hi) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ uint64_t mul_f32x2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t add_f32x2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t sub_f32x2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ float sum_f32x2(uint64_t v) {
+    float a, b;
+    unpack_f32x2(v, a, b);
+    return a + b;
+}
+
+// softplus_fast and softplus_fast_h of a pair, value by value the same
+__device__ __forceinline__ void softplus_fast2(uint64_t z, const SoftplusK& k, uint64_t& h, uint64_t& dh) {
+    float z0, z1, t0, t1, o0, o1, h0, h1;
+    unpack_f32x2(z, z0, z1);
+    unpack_f32x2(mul_f32x2(z, pack_f32x2(k.c1, k.c1)), t0, t1);
+    t0 = fminf(t0, 64.0f);
+    t1 = fminf(t1, 64.0f);
+    const uint64_t e = pack_f32x2(ex2_ftz(t0), ex2_ftz(t1)), one_e = add_f32x2(pack_f32x2(1.0f, 1.0f), e);
+    unpack_f32x2(one_e, o0, o1);
+    dh = mul_f32x2(e, pack_f32x2(rcp_ftz(o0), rcp_ftz(o1)));
+    unpack_f32x2(mul_f32x2(pack_f32x2(lg2_ftz(o0), lg2_ftz(o1)), pack_f32x2(k.c2, k.c2)), h0, h1);
+    h = pack_f32x2(t0 > k.tthr ? z0 : h0, t1 > k.tthr ? z1 : h1);
+}
+__device__ __forceinline__ uint64_t softplus_fast_h2(uint64_t z, const SoftplusK& k) {
+    float z0, z1, t0, t1, o0, o1, h0, h1;
+    unpack_f32x2(z, z0, z1);
+    unpack_f32x2(mul_f32x2(z, pack_f32x2(k.c1, k.c1)), t0, t1);
+    t0 = fminf(t0, 64.0f);
+    t1 = fminf(t1, 64.0f);
+    unpack_f32x2(add_f32x2(pack_f32x2(1.0f, 1.0f), pack_f32x2(ex2_ftz(t0), ex2_ftz(t1))), o0, o1);
+    unpack_f32x2(mul_f32x2(pack_f32x2(lg2_ftz(o0), lg2_ftz(o1)), pack_f32x2(k.c2, k.c2)), h0, h1);
+    return pack_f32x2(t0 > k.tthr ? z0 : h0, t1 > k.tthr ? z1 : h1);
+}
+
 // Column sums of a 32 x 32 block held one row per lane (v[j] = element (lane, j)):
 // recursive-halving exchange, 31 shuffles in total; lane j returns the sum of column j.
 __device__ __forceinline__ float warp_column_sum32(float* v, int lane) {

@@ -170,22 +170,6 @@ __device__ __forceinline__ void scatter_add(float* dst, const float* v) {
 // per (sample, level) keeps thousands of independent loads and atomics in flight,
 // which the tensor-core kernels (one CTA of eight warps per SM) cannot.
 
-// Two float32 lanes in one register pair: fma.rn.f32x2 rounds each lane as fmaf does and
-// takes half the issue slots.
-__device__ __forceinline__ uint64_t pack_f32x2(float lo, float hi) {
-    uint64_t r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
-__device__ __forceinline__ void unpack_f32x2(uint64_t v, float& lo, float& hi) {
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-}
-__device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c) {
-    uint64_t r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-
 // one table row of F fp16 features
 template <int F>
 struct TableRow {
@@ -780,17 +764,21 @@ __global__ void __launch_bounds__(FIELD_THREADS * GROUPS, GROUPS == 1 ? FWD_CTAS
         // epilogue: h = softplus(pre) ; partial head dot ; centre rows keep h in h0c
         const int64_t s = s0 + sl_row;
         const bool keep = row < SPT * EVALS && s < p.Ns && e_row == 0;
-        float part4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        uint64_t part01 = 0ull, part23 = 0ull;          // partial sums of columns j % 4 = 0, 1 and 2, 3
         const SoftplusK spk = softplus_k(p.beta);
 #pragma unroll 1
         for (int c0 = half * 128; c0 < half * 128 + 128; c0 += 32) {
             float v[32];
             umma::tmem_ld32(umma::taddr(tmem, q * 32, c0), v);
 #pragma unroll
-            for (int j = 0; j < 32; ++j) {
-                const float h = softplus_fast_h(v[j], spk);
-                v[j] = h;
-                part4[j & 3] = fmaf(wh_s[c0 + j], h, part4[j & 3]);
+            for (int j = 0; j < 32; j += 4) {
+                const uint64_t h0 = softplus_fast_h2(pack_f32x2(v[j], v[j + 1]), spk);
+                const uint64_t h1 = softplus_fast_h2(pack_f32x2(v[j + 2], v[j + 3]), spk);
+                unpack_f32x2(h0, v[j], v[j + 1]);
+                unpack_f32x2(h1, v[j + 2], v[j + 3]);
+                const ulonglong2 wh = *reinterpret_cast<const ulonglong2*>(wh_s + c0 + j);
+                part01 = fma_f32x2(wh.x, h0, part01);
+                part23 = fma_f32x2(wh.y, h1, part23);
             }
             if (keep) {
                 const int64_t off = s * (int64_t)(p.ld_h0c > 0 ? p.ld_h0c : HID) + c0;
@@ -804,7 +792,7 @@ __global__ void __launch_bounds__(FIELD_THREADS * GROUPS, GROUPS == 1 ? FWD_CTAS
                 }
             }
         }
-        part_s[half * TILE_M + row] = (part4[0] + part4[1]) + (part4[2] + part4[3]);
+        part_s[half * TILE_M + row] = sum_f32x2(part01) + sum_f32x2(part23);
         umma::fence_before_sync();
         group_sync();
         if (tid < SPT * EVALS) {
@@ -1218,49 +1206,54 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_field_bwd(FieldParams p,
             const float df = live ? df_s[(it & 1) * (EVALS * SPT) + row] : 0.0f;
             const bool centre = live && e_row == 0;
             const SoftplusK spk = softplus_k(p.beta);
+            const uint64_t df2 = pack_f32x2(df, df);
             // the next chunk's TMEM load is in flight while this chunk is processed
             uint32_t rn[16];
             umma::tmem_ld16_nowait(umma::taddr(tmem, q * 32, part * 64), rn);
             umma::tmem_ld_wait16(rn);
 #pragma unroll 1
             for (int c0 = part * 64; c0 < part * 64 + 64; c0 += 16) {
-                float v[16];
+                uint64_t v2[8];
 #pragma unroll
-                for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(rn[j]);
+                for (int j = 0; j < 8; ++j) v2[j] = pack_f32x2(__uint_as_float(rn[2 * j]), __uint_as_float(rn[2 * j + 1]));
                 const bool more = c0 + 16 < part * 64 + 64;
                 if (more) umma::tmem_ld16_nowait(umma::taddr(tmem, q * 32, c0 + 16), rn);
-                float dh0[16];
+                uint64_t dh0[8];
                 if (centre) {
-                    const float4* src = reinterpret_cast<const float4*>(dh0_s + sl_row * DH0_LD + c0);
+                    const ulonglong2* src = reinterpret_cast<const ulonglong2*>(dh0_s + sl_row * DH0_LD + c0);
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
-                        const float4 f = src[j];
-                        dh0[4 * j] = f.x; dh0[4 * j + 1] = f.y; dh0[4 * j + 2] = f.z; dh0[4 * j + 3] = f.w;
+                        const ulonglong2 f = src[j];
+                        dh0[2 * j] = f.x;
+                        dh0[2 * j + 1] = f.y;
                     }
                 } else {
 #pragma unroll
-                    for (int j = 0; j < 16; ++j) dh0[j] = 0.0f;
+                    for (int j = 0; j < 8; ++j) dh0[j] = 0ull;
                 }
                 float hc[16];   // d f * h per column: d w_head = sum over rows
+                uint32_t hi[8], lo[8];
+                // pairs of columns: the packed products and sums round as the single ones do and take half
+                // the issue slots (7.12 -> 6.99 ms for 2.1 M samples)
 #pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                    float hval, sg;
-                    softplus_fast(v[j], spk, hval, sg);
-                    v[j] = fmaf(df, wh_s[c0 + j], dh0[j]) * sg;
-                    hc[j] = df * hval;
+                for (int j = 0; j < 8; ++j) {
+                    uint64_t h, sg;
+                    softplus_fast2(v2[j], spk, h, sg);
+                    const uint64_t wh = *reinterpret_cast<const uint64_t*>(wh_s + c0 + 2 * j);
+                    const uint64_t d2 = mul_f32x2(fma_f32x2(df2, wh, dh0[j]), sg);
+                    unpack_f32x2(mul_f32x2(df2, h), hc[2 * j], hc[2 * j + 1]);
+                    float a, b;
+                    unpack_f32x2(d2, a, b);
+                    const __half2 h2 = __floats2half2_rn(a, b);
+                    const float2 back = __half22float2(h2);
+                    unpack_f32x2(sub_f32x2(d2, pack_f32x2(back.x, back.y)), a, b);
+                    const __half2 l2 = __floats2half2_rn(a, b);
+                    hi[j] = *reinterpret_cast<const uint32_t*>(&h2);
+                    lo[j] = *reinterpret_cast<const uint32_t*>(&l2);
                 }
                 {
                     const float colsum = warp_column_sum16(hc, lane);
                     if (lane < 16 && colsum != 0.0f) atomicAdd(&dwh_s[c0 + lane], colsum);
-                }
-                uint32_t hi[8], lo[8];
-#pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    const __half2 h2 = __floats2half2_rn(v[2 * i], v[2 * i + 1]);
-                    const float2 b = __half22float2(h2);
-                    const __half2 l2 = __floats2half2_rn(v[2 * i] - b.x, v[2 * i + 1] - b.y);
-                    hi[i] = *reinterpret_cast<const uint32_t*>(&h2);
-                    lo[i] = *reinterpret_cast<const uint32_t*>(&l2);
                 }
                 if (more) umma::tmem_ld_wait16(rn);
                 umma::tmem_st8(umma::taddr(t_hi(c0 >> 4), q * 32, 0), hi);
