@@ -582,9 +582,11 @@ class FusedField:
     def _in_kernel_w0_grad(self):
         return self.fused_w0_grad and self.K0 <= 64
 
-    def _workspace(self, R, S, Ns, device):
+    def _workspace(self, R, S, Ns, device, train=True):
+        """The buffers of a batch shape.  An evaluation (train False) gets the forward's only, none of
+        them filled (a training step's serve it too)."""
         key = (R, S, Ns, self.K0, self.bg, self.pairs, self.deterministic)
-        if self.ws is not None and self.ws['key'] == key:
+        if self.ws is not None and self.ws['key'] == key and (self.ws['train'] or not train):
             return self.ws
         self.ws = None                      # release the previous shape's buffers first
         # the caller-owned buffers of the field calls, sized by the library
@@ -596,8 +598,12 @@ class FusedField:
         assert rows0 == (Ns + self.spt - 1) // self.spt * self.tile_rows
         f16, f32 = torch.float16, torch.float32
         e = lambda *s, dt=f32: torch.empty(*s, device=device, dtype=dt)  # noqa: E731
+        b = lambda *s, dt=f32: e(*s, dt=dt) if train else None  # noqa: E731  (what only the backward uses)
+        # an activation with its constant-1 column; the inner layers of a chained evaluation stay on chip
+        act = lambda n, w, inner: (self._with_ones(e(n, w + 8, dt=f16), w) if train else  # noqa: E731
+                                   None if inner and self.chain else e(n, w + 8, dt=f16))
         Hc = self.Hc
-        ws = dict(key=key)
+        ws = dict(key=key, train=train)
         # everything a step adds into, in one buffer cleared by one launch: the device flags and
         # loss sums first (all that an evaluation needs), then the gradients in the layouts in
         # which the kernels leave them
@@ -627,21 +633,19 @@ class FusedField:
             ws[name] = arena[at[name]:at[name] + n].view(dt).view(shape)
         gw0x = ws.pop('d_w0')
         ws.update(d_w0=gw0x if dw0 else None, gw0x=gw0x)
-        ws.update(sdf=e(Ns), grad=e(Ns, 3), hess=e(Ns, 3), h0c=self._with_ones(e(Ns, 264, dt=f16), 256),
-                  xc=e(Ns, self.Kc0, dt=f16),
-                  ys=[self._with_ones(e(Ns, Hc + 8, dt=f16), Hc) for _ in range(self.n_rgb_hidden)],
+        ws.update(sdf=e(Ns), grad=e(Ns, 3), hess=e(Ns, 3), h0c=act(Ns, 256, False), xc=e(Ns, self.Kc0, dt=f16),
+                  ys=[act(Ns, Hc, i + 1 < self.n_rgb_hidden) for i in range(self.n_rgb_hidden)],
                   rgbs=e(Ns, 3), rgb=e(R, 3),
-                  weights=e(Ns), d_rgbs=e(Ns, 3), d_sdf=e(Ns), d_grad=e(Ns, 3), d_hess=e(Ns, 3),
-                  dzs=[e(Ns, Hc, dt=f16) for _ in range(2)],
-                  dzs_lo=[e(Ns, Hc, dt=f16) for _ in range(2)] if self.split else None,
-                  dzfeat=e(Ns, 256, dt=f16), dzfeat_lo=e(Ns, 256, dt=f16) if self.split else None,
-                  dxc_tail=e(Ns, 64), d_h0c=e(Ns, 256),
+                  weights=e(Ns), d_rgbs=b(Ns, 3), d_sdf=b(Ns), d_grad=b(Ns, 3), d_hess=b(Ns, 3),
+                  dzs=[b(Ns, Hc, dt=f16) for _ in range(2)],
+                  dzs_lo=[b(Ns, Hc, dt=f16) for _ in range(2)] if self.split else None,
+                  dzfeat=b(Ns, 256, dt=f16), dzfeat_lo=b(Ns, 256, dt=f16) if self.split else None,
+                  dxc_tail=b(Ns, 64), d_h0c=b(Ns, 256),
                   # K0 <= 64: the backward kernel accumulates dW0 itself; otherwise d_pre0 -> k_wgrad
-                  d_pre0=None if self._in_kernel_w0_grad() else e(rows0, 256, dt=f16),
-                  d_pre0_lo=None if self._in_kernel_w0_grad() else e(rows0, 256, dt=f16),
-                  x0ext=e(rows0, 2 * self.K0 + 16, dt=f16), d_enc=e(rows0, self.K0),
-                  d_table_fix=(torch.empty(wsz.d_table_fix_bytes // 8, device=device, dtype=torch.int64)
-                               if self.deterministic else None))
+                  d_pre0=None if self._in_kernel_w0_grad() else b(rows0, 256, dt=f16),
+                  d_pre0_lo=None if self._in_kernel_w0_grad() else b(rows0, 256, dt=f16),
+                  x0ext=e(rows0, 2 * self.K0 + 16, dt=f16), d_enc=b(rows0, self.K0),
+                  d_table_fix=b(wsz.d_table_fix_bytes // 8, dt=torch.int64) if self.deterministic else None)
         if self.pairs:
             # low halves, with the row strides of their hi buffers (the constant-1 column's lo is 0)
             # (a chained forward reads only the field's own: h0c_lo, and the tail columns of xc_lo)
@@ -652,16 +656,16 @@ class FusedField:
         if self.bg:
             Nb = R * self.n_bg
             ws.update(bg_S=e(Nb, BG_S_COLS, dt=f16),
-                      bg_h={i: self._with_ones(e(Nb, 264, dt=f16), 256) for i in (1, 2, 3, 5, 6, 7)},
-                      bg_G=e(Nb, self.Kr0, dt=f16), bg_hr=self._with_ones(e(Nb, Hbr + 8, dt=f16), Hbr),
-                      bg_sigma=e(Nb), bg_rgbs=e(Nb, 3), bg_weights=e(Nb), bg_d_rgbs=e(Nb, 3),
-                      bg_dZ7=torch.zeros(Nb, 272, device=device, dtype=f16), bg_dz_r=e(Nb, Hbr, dt=f16),
-                      bg_dz=[e(Nb, 256, dt=f16) for _ in range(2)],
-                      bg_d_tail=e(Nb, 64) if self.app_dim else None)
+                      bg_h={i: act(Nb, 256, i != 7) for i in (1, 2, 3, 5, 6, 7)},
+                      bg_G=e(Nb, self.Kr0, dt=f16), bg_hr=act(Nb, Hbr, False),
+                      bg_sigma=e(Nb), bg_rgbs=e(Nb, 3), bg_weights=e(Nb), bg_d_rgbs=b(Nb, 3),
+                      bg_dZ7=torch.zeros(Nb, 272, device=device, dtype=f16) if train else None,
+                      bg_dz_r=b(Nb, Hbr, dt=f16), bg_dz=[b(Nb, 256, dt=f16) for _ in range(2)],
+                      bg_d_tail=b(Nb, 64) if self.app_dim else None)
             if self.pairs:
                 # low halves of every background activation that feeds another layer's forward
                 # (or the density head); the colour hidden layer feeds the FP32 head only
-                z = lambda *sh: torch.zeros(*sh, device=device, dtype=f16)  # noqa: E731
+                z = lambda *sh: torch.zeros(*sh, device=device, dtype=f16) if train else None  # noqa: E731
                 # (chained: the encoded columns, and layer 7's input for the density head)
                 ws.update(bg_S_lo=e(Nb, BG_S_COLS, dt=f16),
                           bg_h_lo={i: None if self.chain and i != 7 else e(Nb, 264, dt=f16) for i in (1, 2, 3, 5, 6, 7)},
@@ -716,7 +720,7 @@ class FusedField:
             Ns = R * S
             offs = None
             sample_ray = None
-        ws = self._workspace(R, S, Ns, dev)
+        ws = self._workspace(R, S, Ns, dev, train=not _evaluate)
         scal = self._scalars(dev) if self.dynamic else None
         if scal is not None:
             if _refresh:
@@ -826,10 +830,12 @@ class FusedField:
         ra.d_s_var, ra.loss_sums = _p(ws['d_s_var']), _p(ws['loss_sums'])
         ra.err = _p(ws['err'])
         if self.bg:
-            ra.n_bg, ra.ld_d_bg_pre = self.n_bg, ws['bg_dZ7'].stride(0)
+            ra.n_bg = self.n_bg
             ra.bg_dists, ra.bg_sigma, ra.bg_rgbs = _p(dists_bg), _p(ws['bg_sigma']), _p(ws['bg_rgbs'])
             ra.bg_weights, ra.d_bg_rgbs = _p(ws['bg_weights']), _p(ws['bg_d_rgbs'])
-            ra.d_bg_pre = ws['bg_dZ7'][:, 256:].data_ptr()             # column 256: the density row of layer 7
+            if not _evaluate:
+                ra.ld_d_bg_pre = ws['bg_dZ7'].stride(0)
+                ra.d_bg_pre = ws['bg_dZ7'][:, 256:].data_ptr()         # column 256: the density row of layer 7
         if _evaluate:
             ev = dict(opacity=torch.empty(R, 1, device=dev), gradient=torch.empty(R, 3, device=dev),
                       dist=torch.empty(R, 1, device=dev))
