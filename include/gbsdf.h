@@ -472,6 +472,16 @@ int gbsdf_sampler_coarse(const gbsdf_sampler_args* args, int n, const float* u, 
  * n_fine = 0 the call only merges (the final round). */
 int gbsdf_sampler_round(const gbsdf_sampler_args* args, void* stream);
 
+/* The whole of Model.sample_dists_all (model.py:232-248) on a fused field in one call: coarse
+ * distances and their SDF, n_hierarchy rounds of args->n_fine samples at sharpness 64 * 2^h, the
+ * last merge -- the calls above and gbsdf_sdf_points in order.  Reads R, ld (= n_coarse +
+ * n_hierarchy * n_fine), n_fine, robust, center, ray_unit and dists of args; field carries the SDF
+ * weights (sign as in gbsdf_sdf_points); work: gbsdf_sampler_field_work floats of scratch. */
+int gbsdf_sampler_field(const gbsdf_sampler_args* args, int n_coarse, int n_hierarchy, const float* u, int ldu,
+                        const float* near, const float* far, const gbsdf_field_args* field, float sign, float* work,
+                        int64_t work_floats, void* stream);
+int64_t gbsdf_sampler_field_work(int64_t R, int n_coarse, int n_fine, int n_hierarchy);
+
 /* Weight gradient of a dense layer on the tensor cores (the autograd weight gradient of
  * torch.nn.Linear behind nerf_util.py:187-196, mlp.py:55-69 and modules.py:268-284):
  * dW [N, K] (row stride ldw) = (accumulate ? dW : 0) + (dZ + dZ_lo)[M, N]^T X[M, K].

@@ -26,6 +26,10 @@ int launch_status(const char* what);   // checks cudaGetLastError after a launch
 
 inline cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s); }
 
+// gbsdf_sdf_points with the values in rows of `inner`, `ld` floats apart (inner 0: contiguous); field.cu
+int sdf_points_run(const gbsdf_field_args* params, int64_t M, const float* pts, const float* ax, const float* ay,
+                   const float* az, int nx, int ny, int nz, float sign, float* out, int inner, int ld, cudaStream_t s);
+
 inline bool aligned(const void* p, size_t a) { return (reinterpret_cast<uintptr_t>(p) % a) == 0; }
 
 // Lets kernel k take up to the device's opt-in maximum of dynamic shared memory per

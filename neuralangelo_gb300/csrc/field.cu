@@ -1473,7 +1473,8 @@ struct SdfPointsArgs {
     const float* az;
     int nx, ny, nz;
     float sign;                // +1, or -1 for the mesh's negated field
-    float* out;                // [M]
+    float* out;                // [M], or rows of `inner` values `ld` apart (inner > 0)
+    int inner, ld;
 };
 
 // Warp-specialised, one persistent CTA per SM, two tiles in flight:
@@ -1662,7 +1663,10 @@ __global__ void __launch_bounds__(SP_TPB, 1) k_sdf_points(FieldParams p, SdfPoin
             ps[half * TILE_M + row] = (part4[0] + part4[1]) + (part4[2] + part4[3]);
             named_barrier_sync(2, SP_EPI_WARPS * 32);
             const int64_t m = t * TILE_M + et;
-            if (et < TILE_M && m < q.M) q.out[m] = q.sign * (ps[et] + ps[TILE_M + et] + bhead);
+            if (et < TILE_M && m < q.M) {
+                const int64_t row = q.inner > 0 ? m / q.inner : 0;
+                q.out[row * q.ld + m - row * q.inner] = q.sign * (ps[et] + ps[TILE_M + et] + bhead);
+            }
         }
     }
     umma::fence_before_sync();
@@ -1977,10 +1981,9 @@ extern "C" int gbsdf_field_workspace_size(int64_t Ns, int32_t K0, int32_t taps, 
     return GBSDF_OK;
 }
 
-extern "C" int gbsdf_sdf_points(const gbsdf_field_args* params, int64_t M, const float* pts, const float* ax,
-                                const float* ay, const float* az, int nx, int ny, int nz, float sign, float* out,
-                                void* stream) {
-    clear_error();
+int gbsdf::sdf_points_run(const gbsdf_field_args* params, int64_t M, const float* pts, const float* ax, const float* ay,
+                          const float* az, int nx, int ny, int nz, float sign, float* out, int inner, int ld,
+                          cudaStream_t s) {
     GBSDF_CHECK_ARG(params != nullptr && out != nullptr, "NULL pointer");
     const FieldParams& p = *params;
     if (int st = check_field_weights(p)) return st;
@@ -1988,6 +1991,7 @@ extern "C" int gbsdf_sdf_points(const gbsdf_field_args* params, int64_t M, const
     if (M == 0) return GBSDF_OK;
     SdfPointsArgs q;
     q.M = M; q.pts = pts; q.ax = ax; q.ay = ay; q.az = az; q.nx = nx; q.ny = ny; q.nz = nz; q.sign = sign; q.out = out;
+    q.inner = inner; q.ld = ld;
     if (!pts) {
         GBSDF_CHECK_ARG(ax && ay && az && nx > 0 && ny > 0 && nz > 0 && (int64_t)nx * ny * nz == M,
                         "lattice mode needs axes with nx*ny*nz == M");
@@ -1997,7 +2001,6 @@ extern "C" int gbsdf_sdf_points(const gbsdf_field_args* params, int64_t M, const
     const int64_t ntiles = (M + TILE_M - 1) / TILE_M;
     int64_t grid = num_sms();
     if (grid > ntiles) grid = ntiles;
-    cudaStream_t s = as_stream(stream);
     switch (p.grid.n_features) {
         case 2:
             allow_max_smem(k_sdf_points<2>);
@@ -2013,4 +2016,11 @@ extern "C" int gbsdf_sdf_points(const gbsdf_field_args* params, int64_t M, const
             break;
     }
     return launch_status("sdf_points");
+}
+
+extern "C" int gbsdf_sdf_points(const gbsdf_field_args* params, int64_t M, const float* pts, const float* ax,
+                                const float* ay, const float* az, int nx, int ny, int nz, float sign, float* out,
+                                void* stream) {
+    clear_error();
+    return sdf_points_run(params, M, pts, ax, ay, az, nx, ny, nz, sign, out, 0, 0, as_stream(stream));
 }

@@ -90,17 +90,39 @@ __global__ void __launch_bounds__(SAMPLER_WARPS * 32) k_sampler_round(gbsdf_samp
     const float* d = sd;
     const float* s = ss;
     if (p.n_merge > 0) {
-        // rank sort of the concatenation (ties keep their concatenation order)
+        // stable sort of the concatenation: each entry's rank.  Both parts normally ascend, and then an
+        // entry's rank is its own place plus a binary search in the other part (ties keep the list's
+        // first); a part that does not (bounds with far < near) takes the search over all entries.
         n = cap;
-        for (int i = lane; i < n; i += 32) {
-            const float x = sd[i];
-            int pos = 0;
-            for (int j = 0; j < n; ++j) {
-                const float y = sd[j];
-                pos += (y < x) || (y == x && j < i);
+        bool up = true;
+        for (int i = lane; i + 1 < n; i += 32) up &= i + 1 == p.n_list || sd[i] <= sd[i + 1];
+        if (__all_sync(0xffffffffu, up)) {
+            for (int i = lane; i < n; i += 32) {
+                const float x = sd[i];
+                const bool first = i < p.n_list;
+                int lo = first ? p.n_list : 0, hi = first ? n : p.n_list;
+                const int base = lo;
+                while (lo < hi) {                           // entries of the other part that come before x
+                    const int mid = (lo + hi) >> 1;
+                    const float y = sd[mid];
+                    if (first ? y < x : y <= x) lo = mid + 1;
+                    else hi = mid;
+                }
+                const int pos = (first ? i : i - p.n_list) + lo - base;
+                md[pos] = x;
+                if (with_s) ms[pos] = ss[i];
             }
-            md[pos] = x;
-            if (with_s) ms[pos] = ss[i];
+        } else {
+            for (int i = lane; i < n; i += 32) {
+                const float x = sd[i];
+                int pos = 0;
+                for (int j = 0; j < n; ++j) {
+                    const float y = sd[j];
+                    pos += (y < x) || (y == x && j < i);
+                }
+                md[pos] = x;
+                if (with_s) ms[pos] = ss[i];
+            }
         }
         __syncwarp();
         for (int i = lane; i < n; i += 32) {
@@ -243,6 +265,59 @@ extern "C" int gbsdf_sampler_round(const gbsdf_sampler_args* args, void* stream)
     const int64_t blocks = (p.R + SAMPLER_WARPS - 1) / SAMPLER_WARPS;
     k_sampler_round<<<(unsigned)blocks, SAMPLER_WARPS * 32, smem, as_stream(stream)>>>(p);
     return launch_status("sampler_round");
+}
+
+// floats of the scratch of one run: SDF values [R, N], points of the coarse samples, one round's samples
+static int64_t sampler_work(int64_t R, int nc, int nf, int nh) { return R * ((int64_t)nc + (int64_t)nh * nf + 3ll * nc + 5ll * nf); }
+
+extern "C" int64_t gbsdf_sampler_field_work(int64_t R, int n_coarse, int n_fine, int n_hierarchy) {
+    return sampler_work(R, n_coarse, n_fine, n_hierarchy);
+}
+
+extern "C" int gbsdf_sampler_field(const gbsdf_sampler_args* args, int n_coarse, int n_hierarchy, const float* u, int ldu,
+                                   const float* near, const float* far, const gbsdf_field_args* field, float sign,
+                                   float* work, int64_t work_floats, void* stream) {
+    clear_error();
+    GBSDF_CHECK_ARG(args && field && near && far, "NULL pointer");
+    gbsdf_sampler_args p = *args;
+    const int nf = p.n_fine, nc = n_coarse, N = nc + n_hierarchy * nf;
+    GBSDF_CHECK_ARG(p.R >= 0 && nc >= 1 && n_hierarchy >= 1 && nf >= 1 && nf <= 32 && N <= GBSDF_SAMPLER_MAX_LIST && p.ld >= N,
+                    "%d coarse + %d x %d samples, row stride %d", nc, n_hierarchy, nf, p.ld);
+    if (p.R == 0) return GBSDF_OK;
+    GBSDF_CHECK_ARG(work && work_floats >= sampler_work(p.R, nc, nf, n_hierarchy), "scratch of %lld floats needed",
+                    (long long)sampler_work(p.R, nc, nf, n_hierarchy));
+    cudaStream_t s = as_stream(stream);
+    float* pts = work + p.R * N;
+    float* fine_d = pts + 3 * p.R * nc;
+    float* fine_s = fine_d + p.R * nf;
+    float* fine_pts = fine_s + p.R * nf;
+    // (SDF rows of N values, whatever the distances' stride)
+    GBSDF_CHECK_ARG(p.ld == N, "row stride %d (%d samples)", p.ld, N);
+    p.sdfs = work;
+    p.merge_d = fine_d;
+    p.merge_s = fine_s;
+    p.fine_d = fine_d;
+    p.fine_pts = fine_pts;
+    if (int st = gbsdf_sampler_coarse(&p, nc, u, ldu, near, far, pts, stream)) return st;
+    if (int st = sdf_points_run(field, p.R * nc, pts, nullptr, nullptr, nullptr, 0, 0, 0, sign, p.sdfs, nc, p.ld, s)) return st;
+    p.n_list = nc;
+    for (int h = 0; h < n_hierarchy; ++h) {
+        p.n_merge = h > 0 ? nf : 0;
+        p.inv_s = (float)(64ll << h);
+        if (int st = gbsdf_sampler_round(&p, stream)) return st;
+        p.n_list += p.n_merge;
+        if (h + 1 < n_hierarchy)
+            if (int st = sdf_points_run(field, p.R * nf, fine_pts, nullptr, nullptr, nullptr, 0, 0, 0, sign, fine_s, 0, 0, s))
+                return st;
+    }
+    // the last round's samples: distances only (model.py:240-241)
+    p.n_merge = nf;
+    p.n_fine = 0;
+    p.sdfs = nullptr;
+    p.merge_s = nullptr;
+    p.fine_d = nullptr;
+    p.fine_pts = nullptr;
+    return gbsdf_sampler_round(&p, stream);
 }
 
 extern "C" size_t gbsdf_sampler_args_size(void) { return sizeof(gbsdf_sampler_args); }

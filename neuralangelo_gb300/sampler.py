@@ -29,6 +29,8 @@ class SamplerArgs(ctypes.Structure):
 _lib.register("gbsdf_sampler_args_size", [])
 _lib.register("gbsdf_sampler_coarse", [c_vp, c_i32, c_vp, c_i32, c_vp, c_vp, c_vp, c_vp])
 _lib.register("gbsdf_sampler_round", [c_vp, c_vp])
+_lib.register("gbsdf_sampler_field", [c_vp, c_i32, c_i32, c_vp, c_i32, c_vp, c_vp, c_vp, ctypes.c_float, c_vp,
+                                      ctypes.c_int64, c_vp])
 
 MAX_LIST = 512
 
@@ -76,6 +78,19 @@ class HierarchicalSampler:
             u = u.contiguous().float()
         dists = torch.empty(R, N, **f32)
         if R == 0:
+            return dists
+        from .mesh import FieldSDF
+        if (self.nh > 0 and self.nf > 0 and trace is None and getattr(sdf_fn, "__func__", None) is FieldSDF.points
+                and isinstance(getattr(sdf_fn, "__self__", None), FieldSDF)):
+            # the fused field's own SDF: every launch of the call from one native entry point
+            field = sdf_fn.__self__
+            work = torch.empty(R * (N + 3 * self.nc + 5 * self.nf), **f32)
+            a = SamplerArgs()
+            a.R, a.ld, a.n_fine, a.robust = R, N, self.nf, 1 if self.robust else 0
+            a.center, a.ray_unit, a.dists = _p(center), _p(ray_unit), _p(dists)
+            _lib.call("gbsdf_sampler_field", ctypes.byref(a), self.nc, self.nh, c_vp(_p(u)),
+                      self.nc if u is not None else 0, c_vp(near.data_ptr()), c_vp(far.data_ptr()),
+                      ctypes.byref(field.args), field.sign, c_vp(work.data_ptr()), work.numel(), _lib.stream_ptr(dev))
             return dists
         sdfs = torch.empty(R, N, **f32) if self.nh > 0 else None
         pts = torch.empty(R * self.nc, 3, **f32) if self.nh > 0 else None

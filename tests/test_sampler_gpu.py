@@ -201,3 +201,21 @@ def test_field_sampler_fused_and_plain_sdf_agree():
     assert torch.all(d_fused[:, 1:] >= d_fused[:, :-1])
     close = ((d_fused - d_plain).abs() / span < 1e-3).float().mean().item()
     assert close > 0.95, close
+
+
+@pytest.mark.parametrize("R,nc,nf,nh", [(1, 64, 16, 4), (37, 64, 16, 4), (513, 5, 32, 1), (40, 33, 1, 3), (9, 100, 16, 8)])
+def test_native_field_sampling_equals_the_calls_one_by_one(R, nc, nf, nh):
+    """gbsdf_sampler_field against the same launches issued by the caller, bit for bit: rays that hit,
+    miss and are aimed away (their distances descend, so the merges take the general rank)."""
+    from neuralangelo_gb300.sampler import HierarchicalSampler, field_sdf_fn
+    from tests.test_fused_gpu import build
+    from neuralangelo_gb300.workloads import make_rays, sphere_bounds
+    sdf = field_sdf_fn(build().neural_sdf)
+    b = make_rays(R, 1, seed=R, miss_frac=0.3 if R > 1 else 0.0, device=DEV)
+    near, far, _ = sphere_bounds(b["center"], b["ray_unit"])
+    u = torch.rand(R, nc, device=DEV, generator=torch.Generator(DEV).manual_seed(R))
+    s = HierarchicalSampler(nc, nf, nh)
+    for uu in (None, u):
+        native = s(sdf, b["center"], b["ray_unit"], near, far, u=uu)
+        calls = s(lambda pts: sdf(pts), b["center"], b["ray_unit"], near, far, u=uu)
+        assert torch.equal(native, calls)
