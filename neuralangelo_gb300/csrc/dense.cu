@@ -121,11 +121,11 @@ __global__ void __launch_bounds__(DENSE_TPB, 1) k_dense(const __grid_constant__ 
     if (warp == DENSE_EPI_WARPS) {
         // ---------------- producer: one TMA box (64 columns x 128 rows, 128-byte swizzle) per chunk ----------------
         if (lane == 0) {
-            uint32_t n = 0;
+            int slot = 0;
+            uint32_t use = 0;                                   // (counted: nslots is no constant to divide by)
             bool ok = true;
             for (int64_t t = group; t < ntiles && ok; t += ngroups) {
-                for (int c = 0; c < nchunks; ++c, ++n) {
-                    const uint32_t slot = n % (uint32_t)nslots, use = n / (uint32_t)nslots;
+                for (int c = 0; c < nchunks; ++c) {
                     if (use > 0 && !umma::mbar_wait(&empty[slot], (use - 1) & 1u)) {
                         ok = false;
                         break;
@@ -135,6 +135,10 @@ __global__ void __launch_bounds__(DENSE_TPB, 1) k_dense(const __grid_constant__ 
                     umma::mbar_arrive_expect_tx(&full[slot], CHUNK_BYTES);
                     umma::tma_load_2d(ring + (size_t)slot * CHUNK_BYTES, lo ? (const void*)&tm_xlo : (const void*)&tm_x,
                                       kidx * KCH, (int)(t * TILE_M), &full[slot]);
+                    if (++slot == nslots) {
+                        slot = 0;
+                        ++use;
+                    }
                 }
             }
             if (!ok) flag_timeout(p.err, 1);
@@ -142,43 +146,55 @@ __global__ void __launch_bounds__(DENSE_TPB, 1) k_dense(const __grid_constant__ 
         __syncwarp();
     } else if (warp == DENSE_EPI_WARPS + 1) {
         // ---------------- MMA issue ----------------
-        if (lane == 0) {
-            const uint32_t idesc = umma::idesc_f16(TILE_M, N_TILE);
-            const uint32_t w_addr = umma::smem_u32(w_s), r_addr = umma::smem_u32(ring);
-            uint32_t n = 0;
-            bool ok = true;
-            int i = 0;
-            for (int64_t t = group; t < ntiles && ok; t += ngroups, ++i) {
-                const int buf = i & 1;
-                const uint32_t ub = (uint32_t)(i >> 1);
-                if (ub > 0 && !umma::mbar_wait(&tempty[buf], (ub - 1) & 1u)) {
-                    ok = false;
-                    break;
-                }
+        // The whole warp walks the chunks, one lane polls and the elected one issues: slots and
+        // descriptors are warp-uniform that way.  A lone lane that also divided by the slot count
+        // and rebuilt both descriptors per MMA took longer than its MMAs: 65,536 rows of 256 x 256
+        // softplus as a high and a low half 41.6 -> 38.2 us (N_TILE 128) and 61.5 -> 50.8 (64);
+        // 2.1 M rows are bound by memory and stay at 578 us.
+        const bool leader = umma::elect_one();
+        const uint32_t idesc = umma::idesc_f16(TILE_M, N_TILE);
+        const uint64_t a_desc = umma::make_desc_sw128(umma::smem_u32(ring));
+        const uint64_t w_desc = umma::make_desc(umma::smem_u32(w_s), 128u, (uint32_t)K * 16u);
+        auto wait = [&](uint64_t* bar, uint32_t phase) {
+            return __any_sync(0xffffffffu, lane == 0 && umma::mbar_wait(bar, phase & 1u)) != 0;
+        };
+        int slot = 0;
+        uint32_t use = 0;
+        bool ok = true;
+        int i = 0;
+        for (int64_t t = group; t < ntiles && ok; t += ngroups, ++i) {
+            const int buf = i & 1;
+            const uint32_t ub = (uint32_t)(i >> 1);
+            if (ub > 0) ok = wait(&tempty[buf], ub - 1);
+            if (!ok) break;
+            umma::fence_after_sync();
+            const uint32_t d_tmem = tmem + (uint32_t)(buf * N_TILE);
+            for (int c = 0; c < nchunks; ++c) {
+                ok = wait(&full[slot], use);
+                if (!ok) break;
                 umma::fence_after_sync();
-                const uint32_t d_tmem = tmem + (uint32_t)(buf * N_TILE);
-                for (int c = 0; c < nchunks; ++c, ++n) {
-                    const uint32_t slot = n % (uint32_t)nslots, use = n / (uint32_t)nslots;
-                    if (!umma::mbar_wait(&full[slot], use & 1u)) {
-                        ok = false;
-                        break;
-                    }
-                    umma::fence_after_sync();
-                    const int kidx = p.Xlo ? (c < nk ? c : c - nk) : c;
-                    const int col0 = kidx * KCH, kc = min(KCH, K - col0);
-                    for (int j = 0; j < kc / 16; ++j) {
-                        const uint64_t ad = umma::make_desc_sw128(r_addr + slot * CHUNK_BYTES + j * 32u);
-                        const uint64_t bd = umma::make_desc(w_addr + (uint32_t)(col0 / 16 + j) * 256u, 128u,
-                                                            (uint32_t)K * 16u);
-                        umma::mma_f16(d_tmem, ad, bd, idesc, (c > 0 || j > 0) ? 1u : 0u);
-                    }
+                const int col0 = (c >= nk ? c - nk : c) * KCH, steps = min(KCH, K - col0) / 16;
+                const uint64_t ad = a_desc + (uint64_t)((uint32_t)slot * (CHUNK_BYTES >> 4));
+                const uint64_t bd = w_desc + (uint64_t)(uint32_t)col0;       // 16 columns on: 256 bytes, 16 units
+                const uint32_t acc = c > 0 ? 1u : 0u;
+                if (leader) {
+                    umma::mma_f16(d_tmem, ad, bd, idesc, acc);
+                    if (steps > 1) umma::mma_f16(d_tmem, ad + 2, bd + 16, idesc, 1u);
+                    if (steps > 2) umma::mma_f16(d_tmem, ad + 4, bd + 32, idesc, 1u);
+                    if (steps > 3) umma::mma_f16(d_tmem, ad + 6, bd + 48, idesc, 1u);
                     umma::mma_commit(&empty[slot]);
                 }
-                if (!ok) break;
-                umma::mma_commit(&tfull[buf]);
+                __syncwarp();
+                if (++slot == nslots) {
+                    slot = 0;
+                    ++use;
+                }
             }
-            if (!ok) flag_timeout(p.err, 1);
+            if (!ok) break;
+            if (leader) umma::mma_commit(&tfull[buf]);
+            __syncwarp();
         }
+        if (!ok && leader) flag_timeout(p.err, 1);
         __syncwarp();
     } else {
         // ---------------- epilogue ----------------
@@ -191,7 +207,7 @@ __global__ void __launch_bounds__(DENSE_TPB, 1) k_dense(const __grid_constant__ 
         int i = 0;
         for (int64_t t = group; t < ntiles; t += ngroups, ++i) {
             const int buf = i & 1;
-            if (!umma::mbar_wait(&tfull[buf], (uint32_t)(i >> 1) & 1u)) {
+            if (!__any_sync(0xffffffffu, lane == 0 && umma::mbar_wait(&tfull[buf], (uint32_t)(i >> 1) & 1u))) {
                 if (lane == 0) flag_timeout(p.err, 1);
                 break;
             }
