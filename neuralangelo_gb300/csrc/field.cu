@@ -927,7 +927,9 @@ __global__ void __launch_bounds__(FIELD_THREADS * GROUPS, GROUPS == 1 ? FWD_CTAS
 // (one thread per row would touch 32 cache lines per store instruction); a tile has
 // 126 rows, so the last lane quadrant stores a 30-row box.
 constexpr size_t BWD_SMEM_FLOOR = 120 * 1024;   // > half an SM's shared memory: one CTA per SM
-constexpr int BWD_THREADS = 512;                 // 16 warps: 4 lane quadrants x 4 quarters of the hidden units
+constexpr int BWD_EPI_WARPS = 16;                // 4 lane quadrants x 4 parts of the hidden units
+constexpr int BWD_EPI_THREADS = BWD_EPI_WARPS * 32;
+constexpr int BWD_THREADS = BWD_EPI_THREADS + 32; // and a warp that loads, issues the MMAs and runs the prologue
 constexpr int BWD_STAGE_BYTES = 4096;            // per warp: 32 rows x 128 bytes
 constexpr int DH0_LD = HID + 4;                  // d_h0c rows in shared memory, padded against bank conflicts
 
@@ -960,8 +962,8 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_field_bwd(FieldParams p,
     extern __shared__ __align__(1024) uint8_t smem[];
     const int K0 = p.K0;
     const int KB = K0 + 16;                                     // features hi + tail
-    uint8_t* stage_s = smem;                                    // [16 warps][4 KB] TMA store staging
-    uint8_t* w_s = stage_s + (BWD_THREADS / 32) * BWD_STAGE_BYTES;   // [256 x KB]  w0b: B of MMA1
+    uint8_t* stage_s = smem;                                    // [16][4 KB] TMA store staging, dW0's A operand
+    uint8_t* w_s = stage_s + BWD_EPI_WARPS * BWD_STAGE_BYTES;   // [256 x KB]  w0b: B of MMA1
     uint8_t* a_s0 = w_s + HID * KB * 2;                         // [128 x KB]  features hi | tail
     const int KL = DW ? KB : K0;                                // lo row width (DW: zero-padded)
     uint8_t* a3_s0 = a_s0 + TILE_M * KB * 2;                    // [128 x KL]  features lo
@@ -972,9 +974,11 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_field_bwd(FieldParams p,
     float* df_s = dwh_s + HID;                                  // [2][7][18] d f per evaluation, double-buffered
     float* dh0_s = df_s + TapTile<TAPS>::DF_FLOATS;              // [SPT][DH0_LD] d_h0c of the tile's samples
     uint64_t* mbar = reinterpret_cast<uint64_t*>(dh0_s + SPT * DH0_LD);
-    uint64_t* mbar_lo = mbar + 1;                               // DW: the lo-half dW0 MMAs of a tile
-    uint64_t* mbar_a = mbar + 2;                                // the A tile's TMA loads
-    uint32_t* tslot = reinterpret_cast<uint32_t*>(mbar + 3);
+    uint64_t* mbar_a = mbar + 1;                                // the A tile's TMA loads
+    // DW: hidden units 0-127 written (every epilogue warp); their hi dW0 MMAs done; the lo rows of
+    // units 128-255 written (every epilogue warp)
+    uint64_t *mbar_half = mbar + 2, *mbar_dw = mbar + 3, *mbar_lo = mbar + 4;
+    uint32_t* tslot = reinterpret_cast<uint32_t*>(mbar + 5);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     stage_rows_kmajor(w_s, (const __half*)p.w0b, 0, HID, KB, KB, tid, BWD_THREADS, HID);
@@ -992,8 +996,10 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_field_bwd(FieldParams p,
     }
     if (tid == 0) {
         umma::mbar_init(mbar, 1);
-        umma::mbar_init(mbar_lo, 1);
         umma::mbar_init(mbar_a, 1);
+        umma::mbar_init(mbar_half, BWD_EPI_WARPS);
+        umma::mbar_init(mbar_dw, 1);
+        umma::mbar_init(mbar_lo, BWD_EPI_WARPS);
         umma::fence_mbar_init();
     }
     if (warp == 0) {
@@ -1023,58 +1029,40 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_field_bwd(FieldParams p,
     auto a3_addr = [&](int b) { return umma::smem_u32(a3_buf(b)); };
     bool dw_first = true;                                       // the CTA's first dW0 MMA initialises
     const int64_t ntiles = (p.Ns + SPT - 1) / SPT;
-    const int q = warp & 3, part = warp >> 2;                   // lane quadrant, quarter of the hidden units
+    const bool epi = warp < BWD_EPI_WARPS;                      // an epilogue warp
+    const int q = warp & 3, part = warp >> 2;                   // its lane quadrant and part of the hidden units
+    // its i-th chunk of 16 hidden units: a quarter of them in a row, or (DW) an eighth of units 0-127,
+    // then of 128-255
+    auto chunk = [&](int i) { return DW ? (i >> 1) * 8 + part * 2 + (i & 1) : part * 4 + i; };
     const int row = q * 32 + lane;
     const int e_row = row / SPT, sl_row = row % SPT;
-    uint32_t phase = 0, phase_lo = 0;
+    uint32_t phase = 0;
     float dbh = 0.0f;
     bool ok = true;
 
-    // the prologue runs on warp 1 (lane = sample of the tile), apart from warp 0's MMA issuer
+    // the prologue, on the issuing warp (lane = sample of the tile): per-sample output gradients -> d f
+    // of each evaluation (modules.py:144-156) into df_s[buf], for the next tile under this one's epilogue
     static_assert(TapTile<TAPS>::SPT <= 32, "the prologue's samples fit one warp");
-    const int pl = tid - 32;
-    const bool pl_on = pl >= 0 && pl < SPT;
-    // per-sample output gradients -> d f of each evaluation (modules.py:144-156), for
-    // the next tile while this one is in flight, in three steps that keep the global
-    // loads and the arithmetic off the tile's critical path: the per-sample loads at the
-    // top of the tile, then, while MMA2 runs, the per-ray `outside` flag and the arithmetic
-    // into df_s[buf]
-    struct PrologueIn {
-        float g[3], dg[3], dh[3], n[3], dsdf;
-        int r;
-        bool out;
-    };
-    auto prologue_load = [&](int64_t tt, PrologueIn& in) {
-        const int64_t s = tt * SPT + pl;
-        if (pl_on && s < p.Ns) {
-            in.r = ray_of(p, s);
-#pragma unroll
-            for (int d = 0; d < 3; ++d) {
-                in.g[d] = p.grad[3 * s + d];
-                in.dg[d] = p.d_grad[3 * s + d];
-                in.dh[d] = p.d_hess[3 * s + d];
-            }
-            // normals = g / max(|g|, 1e-12) feed the colour MLP (model.py:167)
-            const float* dn = p.d_xc + s * (int64_t)p.ld_dxc + p.normal_col;
-            in.n[0] = dn[0]; in.n[1] = dn[1]; in.n[2] = dn[2];
-            in.dsdf = p.d_sdf[s];
-        }
-    };
-    auto prologue_ray = [&](int64_t tt, PrologueIn& in) {
-        const int64_t s = tt * SPT + pl;
-        if (pl_on && s < p.Ns) in.out = p.outside && p.outside[in.r];
-    };
-    auto prologue_finish = [&](int64_t tt, const PrologueIn& in, int buf) {
-        if (pl_on) {
-            const int64_t s = tt * SPT + pl;
+    auto prologue = [&](int64_t tt, int buf) {
+        if (!epi && lane < SPT) {
+            const int64_t s = tt * SPT + lane;
             float* dfb = df_s + buf * (EVALS * SPT);
             float df[EVALS];
 #pragma unroll
             for (int e = 0; e < EVALS; ++e) df[e] = 0.0f;
             if (s < p.Ns) {
-                const float g0 = in.g[0], g1 = in.g[1], g2 = in.g[2];
-                const float n0 = in.n[0], n1 = in.n[1], n2 = in.n[2];
-                float dg[3] = {in.dg[0], in.dg[1], in.dg[2]};
+                const int r = ray_of(p, s);
+                float dg[3], dh[3];
+#pragma unroll
+                for (int d = 0; d < 3; ++d) {
+                    dg[d] = p.d_grad[3 * s + d];
+                    dh[d] = p.d_hess[3 * s + d];
+                }
+                const float g0 = p.grad[3 * s], g1 = p.grad[3 * s + 1], g2 = p.grad[3 * s + 2];
+                // normals = g / max(|g|, 1e-12) feed the colour MLP (model.py:167)
+                const float* dn = p.d_xc + s * (int64_t)p.ld_dxc + p.normal_col;
+                const float n0 = dn[0], n1 = dn[1], n2 = dn[2], dsdf = p.d_sdf[s];
+                const bool out = p.outside && p.outside[r];
                 const float len = sqrtf(g0 * g0 + g1 * g1 + g2 * g2);
                 if (len > 1e-12f) {
                     const float inv = 1.0f / len;
@@ -1090,14 +1078,14 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_field_bwd(FieldParams p,
                 if constexpr (TAPS == 6) {
 #pragma unroll
                     for (int d = 0; d < 3; ++d) {
-                        const float a = dg[d] / p.two_eps, b = in.dh[d] / p.eps2;
+                        const float a = dg[d] / p.two_eps, b = dh[d] / p.eps2;
                         df[1 + 2 * d] = a + b;
                         df[2 + 2 * d] = -a + b;
                         hsum += b;
                     }
                 } else {
                     // d H_xx = (dH_x + dH_y + dH_z) / 3; tap i: k_i . dg / (4 e) + d H_xx / (2 e^2)
-                    const float dhxx = (in.dh[0] + in.dh[1] + in.dh[2]) / 3.0f;
+                    const float dhxx = (dh[0] + dh[1] + dh[2]) / 3.0f;
                     const float b = 0.5f * dhxx / p.eps2;
                     const float ax = dg[0] / p.two_eps, ay = dg[1] / p.two_eps, az = dg[2] / p.two_eps;
                     df[1] = ax - ay - az + b;
@@ -1107,11 +1095,11 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_field_bwd(FieldParams p,
                     hsum = dhxx / p.eps2;
                 }
                 // the centre feeds alpha and the Hessian only where it was not overwritten
-                df[0] = in.out ? 0.0f : (in.dsdf - 2.0f * hsum);
+                df[0] = out ? 0.0f : (dsdf - 2.0f * hsum);
             }
 #pragma unroll
             for (int e = 0; e < EVALS; ++e) {
-                dfb[e * SPT + pl] = df[e];
+                dfb[e * SPT + lane] = df[e];
                 dbh += df[e];
             }
         }
@@ -1121,7 +1109,8 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_field_bwd(FieldParams p,
     // are never used) by TMA: one thread, one box per 8-row group and part, straight into
     // the core-matrix layout (rows past the end, and the lo part's zero columns, arrive
     // as zeros); 512 threads' cp.async copies of the same bytes cost them ~2k clocks a tile
-    bool a_pending = false;                         // (thread 0, which issues and waits for these loads)
+    const bool loader = tid == BWD_EPI_THREADS;
+    bool a_pending = false;                         // (the loader, which issues and waits for these loads)
     auto load_a = [&](int64_t tt, int buf) {
         a_pending = true;
         umma::mbar_arrive_expect_tx(mbar_a, (uint32_t)(TILE_M * (KB + KL) * 2));
@@ -1143,8 +1132,8 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_field_bwd(FieldParams p,
         }
         cp_async_commit();
     };
-    auto issue1 = [&](int buf) {                   // warp 0 converged: every call follows a CTA barrier
-        if (warp == 0) {
+    auto issue1 = [&](int buf) {                   // the issuing warp converged
+        if (!epi) {
             if (umma::elect_one()) {
                 if (!umma::mbar_wait(mbar_a, phase_a)) flag_timeout(p.err, 1);   // the A tile's TMA loads
                 a_pending = false;
@@ -1158,12 +1147,9 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_field_bwd(FieldParams p,
         }
     };
     int64_t t = blockIdx.x;
-    PrologueIn pin;
     if (t < ntiles) {
-        prologue_load(t, pin);
-        prologue_ray(t, pin);
-        prologue_finish(t, pin, 0);
-        if (tid == 0) load_a(t, 0);
+        prologue(t, 0);
+        if (loader) load_a(t, 0);
         stage_dh0(t);
         cp_async_wait_all();
         umma::fence_proxy_async_smem();
@@ -1171,12 +1157,13 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_field_bwd(FieldParams p,
     __syncthreads();
     if (t < ntiles) issue1(0);
     int it = 0;
-    // MMA completions: one thread polls the mbarrier and the CTA barrier (a lane shuffle for the
-    // per-warp lo wait) hands on its result
-    for (; t < ntiles && ok; t += gridDim.x, ++it) {
+    // MMA completions: one thread polls the mbarrier and the CTA barrier hands on its result.  A wait that
+    // ran out in one warp alone (ok differs) ends the loop for all at the next barrier.
+    for (; t < ntiles; t += gridDim.x, ++it) {
         const int64_t s0 = t * SPT;
         cp_async_wait_group<0>();                    // this tile's d_h0c rows
-        ok = __syncthreads_and(tid == 0 ? umma::mbar_wait(mbar, phase) : true);   // one poller
+        if (DW && lane == 0) umma::bulk_wait_read0();   // the previous tile's d_enc store has read its rows
+        ok = __syncthreads_and(ok && (loader ? umma::mbar_wait(mbar, phase) : true));   // one poller
         phase ^= 1u;
         if (!ok) {
             flag_timeout(p.err, 1);
@@ -1184,21 +1171,76 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_field_bwd(FieldParams p,
         }
         const int64_t tn = t + gridDim.x;
         const int cb = DW ? (it & 1) : 0, nb = DW ? ((it + 1) & 1) : 0;   // this tile's / the next tile's A
+        const uint32_t par = (uint32_t)it & 1u;      // this tile's parity of the barriers that complete once per tile
         umma::fence_after_sync();
         // the next tile's A tile, under the d_pre epilogue: MMA1 of tile t has completed, and with DW
         // it goes to the other buffer, whose last readers (the previous tile's lo dW0 MMAs) completed
         // before MMA1(t).  (Issued after MMA2 instead, its writes slowed the shared-memory-bound dW0
         // MMAs.)
-        if (tn < ntiles && tid == 0) load_a(tn, nb);
-        if (tn < ntiles) prologue_load(tn, pin);     // consumed under MMA2
-        // (2) d_pre = (d f * w_head + [centre] d_h0c) * softplus'(pre) -> TMEM (hi, lo) and d_pre0
+        if (tn < ntiles && loader) load_a(tn, nb);
+        if (tn < ntiles) prologue(tn, (it + 1) & 1);
         uint8_t* stg = stage_s + warp * BWD_STAGE_BYTES;
+        // d_pre's rows in the staging area: 64 hidden units, 128 rows of 128 bytes, per 16 KB; 128-byte
+        // swizzle: 16-byte unit u of row r sits at u ^ (r & 7)
+        auto stage16 = [&](int c, uint4 u0, uint4 u1) {
+            uint8_t* r = stage_s + (c >> 2) * (4 * BWD_STAGE_BYTES) + row * 128;
+            const int u = (c & 3) * 2;
+            *reinterpret_cast<uint4*>(r + ((u ^ (lane & 7)) * 16)) = u0;
+            *reinterpret_cast<uint4*>(r + (((u + 1) ^ (lane & 7)) * 16)) = u1;
+        };
+        // d_pre's lo half of chunk c, read back from TMEM, into those rows
+        auto stage_lo = [&](int c) {
+            float f[8];
+            umma::tmem_ld8(umma::taddr(t_lo(c), q * 32, 0), f);
+            stage16(c, make_uint4(__float_as_uint(f[0]), __float_as_uint(f[1]), __float_as_uint(f[2]), __float_as_uint(f[3])),
+                    make_uint4(__float_as_uint(f[4]), __float_as_uint(f[5]), __float_as_uint(f[6]), __float_as_uint(f[7])));
+        };
+        // descriptors of this tile's MMA2 and dW0 (warp-uniform values; the elected lane adds constant
+        // multiples of row_step per MMA)
+        const uint64_t row_step = desc_step(2u * KB * 16u);   // 16 rows (dW0's B) / 16 hidden units (MMA2's B)
+        const uint64_t d_stage = umma::make_desc_sw128_mn(umma::smem_u32(stage_s), 16384u, 1024u);
+        const uint32_t id_dw = umma::idesc_f16_mn(TILE_M, KB);
+        const uint64_t d_w = umma::make_desc(w_addr, (uint32_t)KB * 16u, 128u);
+        const uint64_t bx = umma::make_desc(a_addr(cb), KB * 16u, 128u);
+        const uint64_t bx3 = umma::make_desc(a3_addr(cb), KB * 16u, 128u);
+        // d_enc = d_pre * W0e, 32 steps: A = d_pre [128 x 256] in TMEM, lo chunks first (smaller addends),
+        // then hi; B = W0e read MN-major from MMA1's w0b tile: the core matrix of hidden rows 8g..8g+7 and
+        // feature columns 8c..8c+7 sits at g * KB * 16 + c * 128 bytes
+        auto mma2 = [&](int i) {
+            const int ks = i & (HID / 16 - 1);
+            umma::mma_f16_ta(t_enc, i < HID / 16 ? t_lo(ks) : t_hi(ks), d_w + ks * row_step, idesc2, i > 0 ? 1u : 0u);
+        };
+        // dW0[h], 24 steps: += d_pre hi^T [x hi | tail], then d_pre hi^T [x lo | 0], then (the lo rows
+        // staged) d_pre lo^T [x hi | tail].  A (hidden half h = staging blocks 2h, 2h + 1): atoms of 64
+        // units x 8 rows, next 64 units 16 KB on, next 8 rows 1 KB on; B (the tile's rows, MN-major):
+        // next 8 rows KB*16 bytes on, next 8 features 128 bytes on.
+        auto mma_dw = [&](int h, int i) {
+            const int k8 = i & (TILE_M / 16 - 1);
+            umma::mma_f16(t_dw + (uint32_t)(h * KB), d_stage + desc_step(h * 32768 + k8 * 2048),
+                          (i >= TILE_M / 16 && i < 2 * (TILE_M / 16) ? bx3 : bx) + k8 * row_step, id_dw,
+                          (dw_first && i == 0) ? 0u : 1u);
+        };
+        if (DW && !epi) {
+            // units 0-127, under the epilogue of the others: the lo part of MMA2 and the hi dW0 MMAs
+            ok = __any_sync(0xffffffffu, lane == 0 && umma::mbar_wait(mbar_half, par)) != 0;
+            if (ok && umma::elect_one()) {
+                umma::fence_after_sync();
+#pragma unroll
+                for (int i = 0; i < 2 * (TILE_M / 16); ++i) {
+                    if (i < HID / 32) mma2(i);
+                    mma_dw(0, i);
+                }
+                umma::mma_commit(mbar_dw);
+            }
+            __syncwarp();
+        }
+        // (2) d_pre = (d f * w_head + [centre] d_h0c) * softplus'(pre) -> TMEM (hi, lo) and d_pre0
         const CUtensorMap* tm_pre = q == 3 ? &tm_pre30 : &tm_pre32;
         const CUtensorMap* tm_enc = q == 3 ? &tm_enc30 : &tm_enc32;
         const int y0 = (int)(t * TILE_ROWS) + q * 32;
-        if (lane == 0) umma::bulk_wait_read0();      // the previous tile's d_enc store has read the buffer
+        if (!DW && lane == 0) umma::bulk_wait_read0();  // the previous tile's d_enc store has read the buffer
         __syncwarp();
-        {
+        if (epi) {
             // dead rows (past Ns, and rows 126-127) get d f = 0 and no d_h0c: their
             // pre-activations are finite, so their d_pre and head terms come out 0
             const int64_t s = s0 + sl_row;
@@ -1209,15 +1251,16 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_field_bwd(FieldParams p,
             const uint64_t df2 = pack_f32x2(df, df);
             // the next chunk's TMEM load is in flight while this chunk is processed
             uint32_t rn[16];
-            umma::tmem_ld16_nowait(umma::taddr(tmem, q * 32, part * 64), rn);
+            umma::tmem_ld16_nowait(umma::taddr(tmem, q * 32, 16 * chunk(0)), rn);
             umma::tmem_ld_wait16(rn);
 #pragma unroll 1
-            for (int c0 = part * 64; c0 < part * 64 + 64; c0 += 16) {
+            for (int i = 0; i < 4; ++i) {
+                const int c = chunk(i), c0 = 16 * c;
                 uint64_t v2[8];
 #pragma unroll
                 for (int j = 0; j < 8; ++j) v2[j] = pack_f32x2(__uint_as_float(rn[2 * j]), __uint_as_float(rn[2 * j + 1]));
-                const bool more = c0 + 16 < part * 64 + 64;
-                if (more) umma::tmem_ld16_nowait(umma::taddr(tmem, q * 32, c0 + 16), rn);
+                const bool more = i < 3;
+                if (more) umma::tmem_ld16_nowait(umma::taddr(tmem, q * 32, 16 * chunk(i + 1)), rn);
                 uint64_t dh0[8];
                 if (centre) {
                     const ulonglong2* src = reinterpret_cast<const ulonglong2*>(dh0_s + sl_row * DH0_LD + c0);
@@ -1256,41 +1299,41 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_field_bwd(FieldParams p,
                     if (lane < 16 && colsum != 0.0f) atomicAdd(&dwh_s[c0 + lane], colsum);
                 }
                 if (more) umma::tmem_ld_wait16(rn);
-                umma::tmem_st8(umma::taddr(t_hi(c0 >> 4), q * 32, 0), hi);
-                umma::tmem_st8(umma::taddr(t_lo(c0 >> 4), q * 32, 0), lo);
+                umma::tmem_st8(umma::taddr(t_hi(c), q * 32, 0), hi);
+                umma::tmem_st8(umma::taddr(t_lo(c), q * 32, 0), lo);
                 // d_pre0 (hi) into the staging rows; dead samples store zeros (their x0ext
-                // rows are zero too).  128-byte swizzle: 16-byte unit u of row r sits at u ^ (r & 7)
-                const int u = (c0 - part * 64) >> 3;
-                *reinterpret_cast<uint4*>(stg + lane * 128 + ((u ^ (lane & 7)) * 16)) =
-                    make_uint4(hi[0], hi[1], hi[2], hi[3]);
-                *reinterpret_cast<uint4*>(stg + lane * 128 + (((u + 1) ^ (lane & 7)) * 16)) =
-                    make_uint4(hi[4], hi[5], hi[6], hi[7]);
+                // rows are zero too)
+                stage16(c, make_uint4(hi[0], hi[1], hi[2], hi[3]), make_uint4(hi[4], hi[5], hi[6], hi[7]));
+                if (DW && i == 1) {                  // units 0-127 are complete
+                    umma::tmem_wait_st();
+                    umma::fence_proxy_async_smem();
+                    umma::fence_before_sync();
+                    __syncwarp();
+                    if (lane == 0) umma::mbar_arrive(mbar_half);
+                }
+            }
+            if constexpr (DW) {
+                // the lo rows of units 0-127 over their hi rows, which dW0 has read by now
+                umma::tmem_wait_st();
+                ok = __any_sync(0xffffffffu, lane == 0 && umma::mbar_wait(mbar_dw, par)) != 0;
+#pragma unroll
+                for (int i = 0; i < 2; ++i) stage_lo(chunk(i));
             }
         }
         umma::fence_proxy_async_smem();
         __syncwarp();
-        if (!DW && lane == 0) {
+        if (!DW && epi && lane == 0) {
             umma::tma_store_2d(tm_pre, part * 64, y0, stg);
             umma::bulk_commit();
         }
         umma::tmem_wait_st();
-        if (!DW && p.d_pre0_lo) {
+        if (!DW && epi && p.d_pre0_lo) {
             // d_pre's lo half to d_pre0_lo through the same staging rows, read back from TMEM
             // once the hi store has read them (the layer-0 weight gradient needs the pair)
             if (lane == 0) umma::bulk_wait_read0();
             __syncwarp();
 #pragma unroll 1
-            for (int c0 = part * 64; c0 < part * 64 + 64; c0 += 16) {
-                float f[8];
-                umma::tmem_ld8(umma::taddr(t_lo(c0 >> 4), q * 32, 0), f);
-                const int u = (c0 - part * 64) >> 3;
-                *reinterpret_cast<uint4*>(stg + lane * 128 + ((u ^ (lane & 7)) * 16)) =
-                    make_uint4(__float_as_uint(f[0]), __float_as_uint(f[1]), __float_as_uint(f[2]),
-                               __float_as_uint(f[3]));
-                *reinterpret_cast<uint4*>(stg + lane * 128 + (((u + 1) ^ (lane & 7)) * 16)) =
-                    make_uint4(__float_as_uint(f[4]), __float_as_uint(f[5]), __float_as_uint(f[6]),
-                               __float_as_uint(f[7]));
-            }
+            for (int i = 0; i < 4; ++i) stage_lo(chunk(i));
             umma::fence_proxy_async_smem();
             __syncwarp();
             if (lane == 0) {
@@ -1299,54 +1342,32 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_field_bwd(FieldParams p,
             }
         }
         umma::fence_before_sync();
-        __syncthreads();
-        // (3) d_enc = d_pre * W0e  (MMA2: A = d_pre [128 x 256] in TMEM; B = W0e read
-        // MN-major from MMA1's w0b tile: the core matrix of hidden rows 8g..8g+7 and
-        // feature columns 8c..8c+7 sits at g * KB * 16 + c * 128 bytes)
-        {
-            // descriptor bases from converged code (warp-uniform values); the elected lane adds
-            // constant multiples of row_step per MMA
-            const uint64_t row_step = desc_step(2u * KB * 16u);   // 16 rows (dW0's B) / 16 hidden units (MMA2's B)
-            const uint64_t d_stage = umma::make_desc_sw128_mn(umma::smem_u32(stage_s), 16384u, 1024u);
-            const uint32_t id_dw = umma::idesc_f16_mn(TILE_M, KB);
-            const uint64_t d_w = umma::make_desc(w_addr, (uint32_t)KB * 16u, 128u);
-            const uint64_t bx = umma::make_desc(a_addr(cb), KB * 16u, 128u);
-            const uint64_t bx3 = umma::make_desc(a3_addr(cb), KB * 16u, 128u);
-            if (warp == 0 && umma::elect_one()) {      // (warp 0 reconverges below)
-                // MMA2 and (DW) the two dW0 hidden halves go out in turn, each accumulator in its own order
+        ok = __syncthreads_and(ok);
+        if (!ok) {
+            flag_timeout(p.err, 1);
+            break;
+        }
+        // (3) what is left of MMA2 and of dW0, but for the lo rows of units 128-255
+        if (!epi) {
+            if (umma::elect_one()) {
                 umma::fence_after_sync();
 #pragma unroll
-                for (int i = 0; i < 2 * (HID / 16); ++i) {   // d_pre lo chunks first (smaller addends), then hi
-                    const int ks = i & (HID / 16 - 1);
-                    umma::mma_f16_ta(t_enc, i < HID / 16 ? t_lo(ks) : t_hi(ks), d_w + ks * row_step, idesc2,
-                                     i > 0 ? 1u : 0u);
-                    if (DW && i < 2 * (TILE_M / 16)) {
-                        // dW0[h] += d_pre^T [x hi | tail] (i < 8), then += d_pre^T [x lo | 0].
-                        // A (hidden half h = staging parts 2h, 2h + 1): atoms of 64 units x 8 rows, next
-                        // 64 units 16 KB on, next 8 rows 1 KB on; B (the tile's rows, MN-major): next 8
-                        // rows KB*16 bytes on, next 8 features 128 bytes on.
-                        const int k8 = i & (TILE_M / 16 - 1);
-                        const uint64_t bd = (i < TILE_M / 16 ? bx : bx3) + k8 * row_step;
-                        const uint32_t acc0 = (dw_first && i == 0) ? 0u : 1u;
-#pragma unroll
-                        for (int h = 0; h < 2; ++h)
-                            umma::mma_f16(t_dw + (uint32_t)(h * KB), d_stage + desc_step(h * 32768 + k8 * 2048), bd,
-                                          id_dw, acc0);
-                    }
+                for (int i = DW ? HID / 32 : 0; i < 2 * (HID / 16); ++i) {
+                    mma2(i);
+                    if (DW && i - HID / 32 < 2 * (TILE_M / 16)) mma_dw(1, i - HID / 32);
+                    if (DW && i >= 2 * (HID / 16) - TILE_M / 16) mma_dw(0, i - 2 * (HID / 16) + 3 * (TILE_M / 16));
                 }
                 umma::mma_commit(mbar);
             }
+            __syncwarp();                            // the issuing lane rejoins its warp before the barrier
         }
-        if (warp == 0) __syncwarp();                 // the issuing lane rejoins its warp before the barrier
         if constexpr (DW) dw_first = false;
         if (tn < ntiles) {
             // the next tile's d_h0c rows, issued while every thread waits for MMA2 (copies landing
             // under the d_pre epilogue stretch it)
             stage_dh0(tn);                           // every warp has read this tile's d_h0c rows
-            prologue_ray(tn, pin);
-            prologue_finish(tn, pin, (it + 1) & 1);  // the other df buffer, under the MMAs
         }
-        ok = __syncthreads_and(tid == 0 ? umma::mbar_wait(mbar, phase) : true);   // one poller
+        ok = __syncthreads_and(loader ? umma::mbar_wait(mbar, phase) : true);   // one poller
         phase ^= 1u;
         if (!ok) {
             flag_timeout(p.err, 1);
@@ -1354,58 +1375,41 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_field_bwd(FieldParams p,
         }
         umma::fence_after_sync();
         if constexpr (DW) {
-            // dW0[h] += d_pre lo^T [x hi | tail]: the hi MMAs have completed with MMA2, so the
-            // staging rows take d_pre's lo half, read back from TMEM before the next tile's MMA1
+            // dW0[1] += d_pre lo^T [x hi | tail]: its hi MMAs have completed with MMA2, so the staging
+            // rows take d_pre's lo half, read back from TMEM before the next tile's MMA1
             // overwrites it.  The +eps / -eps taps carry large, nearly cancelling d_pre, and a
             // single fp16 rounding of d_pre in dW0 would leave ~1e-3 of it behind.
-#pragma unroll 1
-            for (int c0 = part * 64; c0 < part * 64 + 64; c0 += 16) {
-                float f[8];
-                umma::tmem_ld8(umma::taddr(t_lo(c0 >> 4), q * 32, 0), f);
-                const int u = (c0 - part * 64) >> 3;
-                *reinterpret_cast<uint4*>(stg + lane * 128 + ((u ^ (lane & 7)) * 16)) =
-                    make_uint4(__float_as_uint(f[0]), __float_as_uint(f[1]), __float_as_uint(f[2]),
-                               __float_as_uint(f[3]));
-                *reinterpret_cast<uint4*>(stg + lane * 128 + (((u + 1) ^ (lane & 7)) * 16)) =
-                    make_uint4(__float_as_uint(f[4]), __float_as_uint(f[5]), __float_as_uint(f[6]),
-                               __float_as_uint(f[7]));
-            }
-            umma::fence_proxy_async_smem();
-            umma::fence_before_sync();
-            __syncthreads();
-            const uint64_t row_step = desc_step(2u * KB * 16u);
-            const uint64_t d_stage = umma::make_desc_sw128_mn(umma::smem_u32(stage_s), 16384u, 1024u);
-            const uint32_t id_dw = umma::idesc_f16_mn(TILE_M, KB);
-            const uint64_t bx = umma::make_desc(a_addr(cb), KB * 16u, 128u);
-            if (warp == 0 && umma::elect_one()) {
-                umma::fence_after_sync();
+            if (epi) {
 #pragma unroll
-                for (int ks = 0; ks < TILE_M / 16; ++ks)     // the two hidden halves' chains in turn
+                for (int i = 2; i < 4; ++i) stage_lo(chunk(i));
+                umma::fence_proxy_async_smem();
+                umma::fence_before_sync();
+                __syncwarp();
+                if (lane == 0) umma::mbar_arrive(mbar_lo);
+            } else {
+                ok = __any_sync(0xffffffffu, lane == 0 && umma::mbar_wait(mbar_lo, par)) != 0;
+                if (ok && umma::elect_one()) {
+                    umma::fence_after_sync();
 #pragma unroll
-                    for (int h = 0; h < 2; ++h)
-                        umma::mma_f16(t_dw + (uint32_t)(h * KB), d_stage + desc_step(h * 32768 + ks * 2048),
-                                      bx + ks * row_step, id_dw, 1u);
-                umma::mma_commit(mbar_lo);
+                    for (int i = 2 * (TILE_M / 16); i < 3 * (TILE_M / 16); ++i) mma_dw(1, i);
+                    if (tn >= ntiles) umma::mma_commit(mbar);      // else MMA1's commit covers them
+                }
+                __syncwarp();
+                // D1 is free: MMA2 has read d_pre, the warps its lo half
+                if (ok && tn < ntiles) issue1(nb);
             }
-            if (warp == 0) __syncwarp();
         }
-        if (DW && tn < ntiles) issue1(nb);           // D1 is free: MMA2 has read d_pre
         // (4) d_enc rows to global for k_field_scatter: 16-column chunks dealt in turn
         // to the four warps of a lane quadrant (K0 <= 128: at most two per warp, one
         // 2 KB half of the staging buffer each; 64-byte swizzle: unit j of row r at j ^ ((r >> 1) & 3))
-        if (lane == 0) umma::bulk_wait_read0();      // the d_pre0 store (or, DW, dW0's MMAs) has read it
-        if constexpr (DW) {
-            // the lo dW0 MMAs read the staging rows: wait for them before d_enc goes through
-            // (a timed-out wait skips this warp's stores; the tile's closing barrier ends the loop)
-            ok = __shfl_sync(0xffffffffu, lane == 0 ? (int)umma::mbar_wait(mbar_lo, phase_lo) : 0, 0) != 0;
-            phase_lo ^= 1u;
-            if (!ok && lane == 0) flag_timeout(p.err, 1);
-        }
+        // With DW (one chunk) they go through the rows of units 0-127, 2 KB per warp: dW0's MMAs have
+        // read those, and are about to read the others.
+        if (!DW && lane == 0) umma::bulk_wait_read0();   // the d_pre0 store has read the buffer
         __syncwarp();
-        for (int c0 = part * 16, i = 0; ok && c0 < K0; c0 += 64, ++i) {
+        for (int c0 = part * 16, i = 0; epi && c0 < K0; c0 += 64, ++i) {
             float v[16];
             umma::tmem_ld16(umma::taddr(t_enc, q * 32, c0), v);
-            uint8_t* eb = stg + i * 2048;
+            uint8_t* eb = DW ? stage_s + warp * 2048 : stg + i * 2048;
 #pragma unroll
             for (int j = 0; j < 4; ++j)
                 *reinterpret_cast<float4*>(eb + lane * 64 + ((j ^ ((lane >> 1) & 3)) * 16)) =
@@ -1418,18 +1422,26 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_field_bwd(FieldParams p,
             }
         }
         umma::fence_before_sync();
-        ok = __syncthreads_and(ok);   // the TMEM accumulator of tile t read; tile tn's A tile and d f in place
-        if (ok && !DW && tn < ntiles) issue1(nb);
+        if constexpr (!DW) {
+            __syncthreads();                         // the TMEM accumulator of tile t read; tile tn's A tile and d f in place
+            if (tn < ntiles) issue1(nb);
+        }                                            // (DW: the next tile's first barrier says so)
+    }
+    if (DW && blockIdx.x < ntiles) {                 // the last tile's lo dW0 MMAs
+        const bool done = ok && (loader ? umma::mbar_wait(mbar, phase) : true);
+        if (!done) flag_timeout(p.err, 1);
+        ok = __syncthreads_and(done);
+        umma::fence_after_sync();
     }
     cp_async_wait_all();
-    if (tid == 0 && a_pending && !umma::mbar_wait(mbar_a, phase_a)) flag_timeout(p.err, 1);   // a load left in flight
+    if (loader && a_pending && !umma::mbar_wait(mbar_a, phase_a)) flag_timeout(p.err, 1);   // a load left in flight
     if (lane == 0) umma::bulk_wait0();               // this warp's TMA stores have completed
     umma::fence_before_sync();
     __syncthreads();
     if constexpr (DW) {
         // the CTA's dW0 (complete: the last tile's lo MMAs were waited for): warps with part 2h, 2h + 1
         // read hidden half h, one half of its KB columns each
-        if (!dw_first && ok) {
+        if (!dw_first && ok && epi) {
             umma::fence_after_sync();
             const int h = part >> 1, half_cols = KB / 2, cbeg = (part & 1) * half_cols;
             float* dst = p.d_w0 + (int64_t)(h * 128 + q * 32 + lane) * KB;
@@ -1688,9 +1700,9 @@ static size_t fwd_smem(int K0, int app_dim, int groups) {
 template <int TAPS>
 static size_t bwd_smem(int K0, bool dw) {
     const size_t KB = (size_t)K0 + 16;
-    const size_t need = (size_t)(BWD_THREADS / 32) * BWD_STAGE_BYTES + (size_t)HID * KB * 2 +
+    const size_t need = (size_t)BWD_EPI_WARPS * BWD_STAGE_BYTES + (size_t)HID * KB * 2 +
                         (size_t)TILE_M * (KB + (dw ? KB : K0)) * 2 * (dw ? 2 : 1) +
-                        (2 * HID + TapTile<TAPS>::DF_FLOATS + TapTile<TAPS>::SPT * DH0_LD) * 4 + 32;
+                        (2 * HID + TapTile<TAPS>::DF_FLOATS + TapTile<TAPS>::SPT * DH0_LD) * 4 + 48;
     return need > BWD_SMEM_FLOOR ? need : BWD_SMEM_FLOOR;
 }
 
