@@ -1,8 +1,8 @@
 """Launch-shape autotuner of the fused step (project-written).
 
 The fused step's kernels have launch shapes that do not change their results but do change
-their speed with the workload: the table scatter's corners per pass (register use against
-resident warps), the field forward's CTAs per SM, and each dense layer shape's N tile and
+their speed with the workload: the table scatter's samples per thread (fewer atomics against
+more threads), the field forward's CTAs per SM, and each dense layer shape's N tile and
 pipeline depth.  ``StepTuner.tune(batch)`` runs one eager step to build the workspace, then
 re-issues each of those calls on the step's own buffers for every candidate shape, times them
 with CUDA events on the launching stream, and keeps the fastest.  Choices are cached per

@@ -105,16 +105,6 @@ __device__ __forceinline__ float to_unit(float p) { return __fmul_rn(__fadd_rn(p
 // ---------------------------------------------------------------------------
 // numerics shared with the reference's activations
 
-// torch.nn.functional.softplus(x, beta, threshold=20)
-__device__ __forceinline__ float softplus_beta(float x, float beta) {
-    const float bx = x * beta;
-    return bx > 20.0f ? x : log1pf(expf(bx)) / beta;
-}
-// d softplus / dx = sigmoid(beta*x) (1 above the threshold)
-__device__ __forceinline__ float softplus_grad(float x, float beta) {
-    const float bx = x * beta;
-    return bx > 20.0f ? 1.0f : 1.0f / (1.0f + expf(-bx));
-}
 __device__ __forceinline__ float sigmoidf_(float x) { return 1.0f / (1.0f + expf(-x)); }
 
 // MUFU approximations with subnormals flushed to zero (PTX ex2/lg2/rcp .approx.ftz):
@@ -153,14 +143,6 @@ __device__ __forceinline__ SoftplusK softplus_k(float beta) {
     k.c2 = 0.6931471805599453f / beta;
     k.tthr = 20.0f * 1.4426950408889634f;
     return k;
-}
-__device__ __forceinline__ void softplus_fast(float z, const SoftplusK& k, float& h, float& dh) {
-    const float t = fminf(z * k.c1, 64.0f);
-    const float e = ex2_ftz(t);
-    const float one_e = 1.0f + e;
-    dh = e * rcp_ftz(one_e);
-    const float hl = lg2_ftz(one_e) * k.c2;
-    h = t > k.tthr ? z : hl;
 }
 __device__ __forceinline__ float softplus_fast_h(float z, const SoftplusK& k) {
     const float t = fminf(z * k.c1, 64.0f);
@@ -204,7 +186,7 @@ __device__ __forceinline__ float sum_f32x2(uint64_t v) {
     return a + b;
 }
 
-// softplus_fast and softplus_fast_h of a pair, value by value the same
+// softplus and its derivative, or softplus alone, of a pair; softplus as softplus_fast_h, value by value
 __device__ __forceinline__ void softplus_fast2(uint64_t z, const SoftplusK& k, uint64_t& h, uint64_t& dh) {
     float z0, z1, t0, t1, o0, o1, h0, h1;
     unpack_f32x2(z, z0, z1);
@@ -226,22 +208,6 @@ __device__ __forceinline__ uint64_t softplus_fast_h2(uint64_t z, const SoftplusK
     unpack_f32x2(add_f32x2(pack_f32x2(1.0f, 1.0f), pack_f32x2(ex2_ftz(t0), ex2_ftz(t1))), o0, o1);
     unpack_f32x2(mul_f32x2(pack_f32x2(lg2_ftz(o0), lg2_ftz(o1)), pack_f32x2(k.c2, k.c2)), h0, h1);
     return pack_f32x2(t0 > k.tthr ? z0 : h0, t1 > k.tthr ? z1 : h1);
-}
-
-// Column sums of a 32 x 32 block held one row per lane (v[j] = element (lane, j)):
-// recursive-halving exchange, 31 shuffles in total; lane j returns the sum of column j.
-__device__ __forceinline__ float warp_column_sum32(float* v, int lane) {
-#pragma unroll
-    for (int h = 16; h >= 1; h >>= 1) {
-        const bool upper = (lane & h) != 0;
-#pragma unroll
-        for (int i = 0; i < h; ++i) {
-            const float send = upper ? v[i] : v[i + h];
-            const float keep = upper ? v[i + h] : v[i];
-            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, h);
-        }
-    }
-    return v[0];
 }
 
 // Column sums of a 32 x 16 block held one row per lane (v[j] = element (lane, j)):

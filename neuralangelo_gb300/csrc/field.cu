@@ -11,9 +11,9 @@
 // of a 128-row tcgen05 tile.  Row r holds evaluation e = r / 18 of sample r % 18:
 // e = 0 centre, 1 +x, 2 -x, 3 +y, 4 -y, 5 +z, 6 -z.  With 4 taps (the tetrahedral
 // stencil, modules.py:157-175) a tile is 25 samples x 5 evaluations = 125 rows.  The hash-grid features of
-// the active levels are gathered straight into the shared-memory A tile
-// (fp16, K-major core-matrix layout); W0's encoding columns are resident; the
-// three position columns, bias, softplus and the SDF head run in fp32 in the
+// the active levels are gathered into rows of global memory (x0ext: fp16 hi,
+// position/bias tail, fp16 lo) by a kernel of its own and loaded from there by TMA;
+// layer 0's weights are resident; softplus and the SDF head run in fp32 in the
 // epilogue, so SDF values and the tap differences keep fp32 accuracy.
 #include "dense.cuh"
 #include "tma.cuh"
@@ -73,39 +73,6 @@ __device__ __forceinline__ void eval_point(const float* c, int e, float eps, flo
     }
 }
 
-// Gather the active levels of one (row, level) pair into the A tile.
-template <int F>
-__device__ __forceinline__ void gather_level(const FieldParams& p, const float* xu, int l, float* out) {
-    const LevelDesc d = level_desc(p.grid, l);
-    uint32_t bx, by, bz;
-    float fx, fy, fz;
-    grid_pos(d.scale, xu[0], bx, fx);
-    grid_pos(d.scale, xu[1], by, fy);
-    grid_pos(d.scale, xu[2], bz, fz);
-#pragma unroll
-    for (int f = 0; f < F; ++f) out[f] = 0.0f;
-#pragma unroll
-    for (int c = 0; c < 8; ++c) {
-        const uint32_t idx = grid_index(d, bx + (c & 1), by + ((c >> 1) & 1), bz + ((c >> 2) & 1));
-        const float w = corner_weight(c, fx, fy, fz);
-        const __half* row = (const __half*)p.table + (d.offset + idx) * F;
-        float v[F];
-        if constexpr (F == 8) {
-            load_half8(row, v);
-        } else if constexpr (F == 4) {
-            const uint2 u = __ldg(reinterpret_cast<const uint2*>(row));
-            const __half2* h = reinterpret_cast<const __half2*>(&u);
-            const float2 a = __half22float2(h[0]), b = __half22float2(h[1]);
-            v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
-        } else {
-#pragma unroll
-            for (int f = 0; f < F; ++f) v[f] = __half2float(row[f]);
-        }
-#pragma unroll
-        for (int f = 0; f < F; ++f) out[f] = fmaf(w, v[f], out[f]);
-    }
-}
-
 template <int F>
 __device__ __forceinline__ void write_half_row(uint8_t* dst, const float* v) {
     if constexpr (F == 8) {
@@ -154,10 +121,7 @@ __global__ void k_fixed_to_table(int64_t n, const unsigned long long* __restrict
 
 template <int F>
 __device__ __forceinline__ void scatter_add(float* dst, const float* v) {
-    if constexpr (F == 8) {
-        atomicAdd(reinterpret_cast<float4*>(dst), make_float4(v[0], v[1], v[2], v[3]));
-        atomicAdd(reinterpret_cast<float4*>(dst) + 1, make_float4(v[4], v[5], v[6], v[7]));
-    } else if constexpr (F == 4) {
+    if constexpr (F == 4) {
         atomicAdd(reinterpret_cast<float4*>(dst), make_float4(v[0], v[1], v[2], v[3]));
     } else {
 #pragma unroll

@@ -1,5 +1,5 @@
 // Exclusive int64 scan with caller workspace (block scans, recursive on the block
-// sums), shared by the mesh kernels.  Everything here has internal linkage, so
+// sums), for the mesh output.  Everything here has internal linkage, so
 // each translation unit that includes it gets its own copy.
 #pragma once
 
