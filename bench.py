@@ -521,7 +521,7 @@ def main():
     # the dense layers, weight gradients and colour head: their algorithmic bytes as each call
     # reported them (fused.py: operand and output rows, hi + lo halves counted); their tensor
     # work is far below their HBM floor
-    for name in ("gbsdf_dense", "gbsdf_wgrad", "gbsdf_rgb_head_fwd", "gbsdf_rgb_head_bwd"):
+    for name in ("gbsdf_mlp_chain", "gbsdf_dense", "gbsdf_wgrad", "gbsdf_rgb_head_fwd", "gbsdf_rgb_head_bwd"):
         if name in kbytes and name in ksum:
             work[name] = (kbytes[name] / ksum[name][0], 0)
     tensor_peak = peaks.get("bf16_tflops_sustained", 1700.0)
