@@ -895,7 +895,11 @@ __global__ void __launch_bounds__(FIELD_THREADS * GROUPS, GROUPS == 1 ? FWD_CTAS
 constexpr size_t BWD_SMEM_FLOOR = 120 * 1024;   // > half an SM's shared memory: one CTA per SM
 constexpr int BWD_EPI_WARPS = 16;                // 4 lane quadrants x 4 parts of the hidden units
 constexpr int BWD_EPI_THREADS = BWD_EPI_WARPS * 32;
-constexpr int BWD_THREADS = BWD_EPI_THREADS + 32; // and a warp that loads, issues the MMAs and runs the prologue
+// and a warp that loads, issues the MMAs and runs the prologue: as an epilogue warp's extra work those
+// held the other fifteen up.  With it and the halves below 6.49 ms for 2.1 M samples at K0 = 64, 6.99
+// with one epilogue warp issuing everything after the whole epilogue (17 warps leave 96 registers
+// a thread, which the epilogue just fits).
+constexpr int BWD_THREADS = BWD_EPI_THREADS + 32;
 constexpr int BWD_STAGE_BYTES = 4096;            // per warp: 32 rows x 128 bytes
 constexpr int DH0_LD = HID + 4;                  // d_h0c rows in shared memory, padded against bank conflicts
 
@@ -907,12 +911,18 @@ constexpr int DH0_LD = HID + 4;                  // d_h0c rows in shared memory,
 //   * The dW0 MMAs read both operands MN-major: A = the d_pre hi rows of the staging
 //     buffers (128-byte swizzle atoms of 64 hidden units x 8 rows), B = the tile's x0ext rows.
 //   * The feature tile is double-buffered: the next tile's load may not overwrite what
-//     dW0 reads.  dW0 goes before MMA2, so MMA2's completion also frees the staging rows.
+//     dW0 reads.
+//   * Hidden units 0-127 come first: the lo part of MMA2 and the hi dW0 MMAs of them run under the
+//     epilogue of units 128-255, then their lo rows replace the hi rows in the staging area, so that
+//     the tile's second phase is MMA2's rest, the other half's hi dW0 and this half's lo dW0.  Every
+//     accumulator takes its products in one order: MMA2 lo then hi, dW0 hi x hi, hi x lo, lo x hi.
+//   * d_enc leaves through the rows of units 0-127, whose MMAs are done by then, while the lo dW0 MMAs of
+//     units 128-255 read theirs.
 //   * The lo feature rows are K0 + 16 columns wide, the last 16 zero, so that the lo dW0
 //     MMAs have the hi MMAs' shape (MMAs into one accumulator are ordered when their
 //     shapes agree).
-//   * MMA1 of the next tile is issued as soon as MMA2 has completed (D1 is free then),
-//     under the d_enc epilogue.
+//   * MMA1 of the next tile is issued as soon as MMA2 has completed and the warps have read d_pre's lo
+//     half (D1 is free then), under the d_enc epilogue.
 //   * Each CTA adds its dW0 into d_w0 with atomics at the end.
 template <int F, bool DW, int TAPS>
 __global__ void __launch_bounds__(BWD_THREADS, 1) k_field_bwd(FieldParams p,
